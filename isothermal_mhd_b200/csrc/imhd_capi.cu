@@ -319,6 +319,7 @@ int imhd_create(const imhd_config* cfg, imhd_box** out) {
     x->esz = c.precision == 64 ? 8 : 4;
     imhd::init_rec(x->rec, c.nx, c.ny, c.nz, c.npass, c.riemann, c.recon, c.sound_speed, c.cour, c.edot, c.dt_turb,
                    c.protect);
+    imhd::one_box_segments(x->rec, x->esz);
     imhd::BatchDev& b = x->b;
     b.precision = c.precision;
     size_t N = (size_t)x->rec.n;

@@ -76,10 +76,11 @@ __device__ __forceinline__ void decode_cell(int local, const Dims& dm, int tws, 
 
 // kKindCellZ decomposition: the same tiles per z segment of kSegZ planes
 // (a compile-time length: the unrolled z loops are measurably faster with
-// it); the thread's column is k0 <= k < k1 (a single box launches a 3D grid
-// (nbx, nby, nseg)).
+// it), or of 1 << segzs planes (SHORT: a single box too small to fill the GPU
+// with kSegZ-plane columns, see one_box_segments); the thread's column is
+// k0 <= k < k1 (a single box launches a 3D grid (nbx, nby, nseg)).
 // Callers test i < nx and j < ny.
-template <bool ONE>
+template <bool ONE, bool SHORT = false>
 __device__ __forceinline__ void decode_cellz(int local, const Dims& dm, int tws, int segzs, int& i, int& j, int& k0,
                                              int& k1) {
     const int tw = 1 << tws, th = kBX >> tws;
@@ -96,9 +97,9 @@ __device__ __forceinline__ void decode_cellz(int local, const Dims& dm, int tws,
         j = (rest % nby) * th + ly;
         seg = rest / nby;
     }
-    (void)segzs;
-    k0 = seg * kSegZ;
-    k1 = min(k0 + kSegZ, dm.nz);
+    const int len = SHORT ? 1 << segzs : kSegZ;
+    k0 = seg * len;
+    k1 = min(k0 + len, dm.nz);
 }
 
 __device__ __forceinline__ int wrap_up(int i, int n) { return (i + 1 == n) ? 0 : i + 1; }
@@ -218,7 +219,7 @@ __device__ __forceinline__ void protection_flux(const T* uL, const T* uR, T cs, 
 // FP32 occupancy, measured at 512^3: five blocks per SM for the Roe solver
 // (96 registers; fewer registers spill more than the extra warps return), six
 // for HLLD and HLLE (80 registers, 3.9 -> 3.7 ms).
-template <class T, int SCHEME, bool ONE>
+template <class T, int SCHEME, bool ONE, bool SHORT = false>
 __global__ void __launch_bounds__(kBX, sizeof(T) == 4 ? (scheme_solver(SCHEME) % 3 == 1 ? 5 : 6) : 1)
 k_pred_flux(BatchArgs ba) {
     constexpr int SOLVER = scheme_solver(SCHEME);
@@ -232,7 +233,7 @@ k_pred_flux(BatchArgs ba) {
     const T cs = (T)rp.cs, asqr = (T)(rp.cs * rp.cs);
     unsigned long long* smax_slots = sc->smax_slots;
     int i, j, k0, k1;
-    decode_cellz<ONE>(local, dm, rp.tws, rp.segzs, i, j, k0, k1);
+    decode_cellz<ONE, SHORT>(local, dm, rp.tws, rp.segzs, i, j, k0, k1);
     const bool valid = i < dm.nx && j < dm.ny;
     T smax = T(0);
     if (valid) {
@@ -675,7 +676,7 @@ __device__ __forceinline__ CellEV<T> cell_ev(const T* __restrict__ S, int n, int
 // they gained, 2.2 -> 2.4 ms at 512^3); eight in a table, whose small boxes
 // leave the loads less overlapped (the batched workload 4.48 -> 4.70e9
 // cell-updates/s).
-template <class T, bool ONE, bool PROT = false>
+template <class T, bool ONE, bool PROT = false, bool SHORT = false>
 __global__ void __launch_bounds__(kBX, sizeof(T) == 4 ? (ONE ? 6 : 8) : 1) k_corner_emf(BatchArgs ba,
                                                                                        int half_step_state) {
     int local;
@@ -686,7 +687,7 @@ __global__ void __launch_bounds__(kBX, sizeof(T) == 4 ? (ONE ? 6 : 8) : 1) k_cor
     const T* __restrict__ F = (const T*)(PROT ? rp.Fp : rp.F);
     T* __restrict__ E = (T*)(PROT ? rp.Ep : rp.E);
     int i, j, k0, k1;
-    decode_cellz<ONE>(local, dm, rp.tws, rp.segzs, i, j, k0, k1);
+    decode_cellz<ONE, SHORT>(local, dm, rp.tws, rp.segzs, i, j, k0, k1);
     if (i >= dm.nx || j >= dm.ny) return;
     const int n = dm.n;
     const int plane = dm.nx * dm.ny;
@@ -852,7 +853,7 @@ __device__ __forceinline__ bool update_by_tma(const BoxRec& r) {
 // the "k-1" values of plane k+1 and are carried instead of reloaded.
 // ZR: some box of the table restricts its maxima to a z range (slabs); the
 // other instantiation has no per-plane test on the hot path.
-template <class T, bool ONE, bool ZR>
+template <class T, bool ONE, bool ZR, bool SHORT = false>
 __global__ void __launch_bounds__(kBX, sizeof(T) == 4 ? 6 : 1) k_update(BatchArgs ba, double dt_scale, int final_stage) {
     int local;
     const BoxRec rp = resolve<ONE>(ba, kKindCellZ, local);
@@ -872,7 +873,7 @@ __global__ void __launch_bounds__(kBX, sizeof(T) == 4 ? 6 : 1) k_update(BatchArg
     unsigned long long* floor_hits = &sc->floor_hits;
     unsigned int* status = &sc->status;
     int i, j, k0, k1;
-    decode_cellz<ONE>(local, dm, rp.tws, rp.segzs, i, j, k0, k1);
+    decode_cellz<ONE, SHORT>(local, dm, rp.tws, rp.segzs, i, j, k0, k1);
     const bool valid = i < dm.nx && j < dm.ny;
     double cmax = 0.0;
     if (valid) {
@@ -1057,7 +1058,8 @@ __global__ void __launch_bounds__(kTmaTile, sizeof(T) == 4 ? 6 : 1)
         seg = rest / nby;
     }
     const int i = i0 + lx, j = j0 + ly;
-    const int k0 = seg * kSegZ, k1 = min(k0 + kSegZ, dm.nz);
+    const int len = ONE ? 1 << rp.segzs : kSegZ;
+    const int k0 = seg * len, k1 = min(k0 + len, dm.nz);
     const int n = dm.n, plane = dm.nx * dm.ny;
     const int jm = wrap_dn(j, dm.ny);
     const T dtdx = (T)(dt_scale * sc->dt / rp.dx);
@@ -1440,7 +1442,7 @@ __device__ __forceinline__ T vel_of(const T* __restrict__ S, int n, int c, int c
 // cell: the same operands).  The neighbour loads are
 // latency-bound, so FP32 with up to four scalars runs eight blocks per SM
 // (64 registers).
-template <class T, bool ONE, int NP>
+template <class T, bool ONE, int NP, bool SHORT = false>
 __global__ void __launch_bounds__(kBX, (sizeof(T) == 4 && NP <= 4) ? 8 : 1) k_passive_pred(BatchArgs ba) {
     int local;
     const BoxRec rp = resolve<ONE>(ba, kKindCellZ, local);
@@ -1452,7 +1454,7 @@ __global__ void __launch_bounds__(kBX, (sizeof(T) == 4 && NP <= 4) ? 8 : 1) k_pa
     T* __restrict__ SH = (T*)rp.SH;
     const double dx = rp.dx;
     int i, j, k0, k1;
-    decode_cellz<ONE>(local, dm, rp.tws, rp.segzs, i, j, k0, k1);
+    decode_cellz<ONE, SHORT>(local, dm, rp.tws, rp.segzs, i, j, k0, k1);
     if (i >= dm.nx || j >= dm.ny) return;
     const int n = dm.n;
     const int plane = dm.nx * dm.ny;
@@ -1529,7 +1531,7 @@ __device__ __forceinline__ T vtavg(const T* __restrict__ S0, const T* __restrict
 // flux through the lower z face (the upper face's of the previous cell).
 // Eight blocks per SM in FP32 with up to four scalars, as k_passive_pred
 // (a few spilled values cost less than the lost occupancy).
-template <class T, bool ONE, int NP>
+template <class T, bool ONE, int NP, bool SHORT = false>
 __global__ void __launch_bounds__(kBX, (sizeof(T) == 4 && NP <= 4) ? 8 : 1) k_passive_corr(BatchArgs ba) {
     int local;
     const BoxRec rp = resolve<ONE>(ba, kKindCellZ, local);
@@ -1546,7 +1548,7 @@ __global__ void __launch_bounds__(kBX, (sizeof(T) == 4 && NP <= 4) ? 8 : 1) k_pa
     const T* __restrict__ mbnd = (const T*)rp.mbnd;
     const int plane_stride = rp.plane_stride;
     int i, j, k0, k1;
-    decode_cellz<ONE>(local, dm, rp.tws, rp.segzs, i, j, k0, k1);
+    decode_cellz<ONE, SHORT>(local, dm, rp.tws, rp.segzs, i, j, k0, k1);
     if (i >= dm.nx || j >= dm.ny) return;
     const int n = dm.n;
     const int plane = dm.nx * dm.ny;
@@ -1682,7 +1684,7 @@ __global__ void __launch_bounds__(kTmaTile, 8) k_passive_corr_tma(BatchArgs ba) 
     const int t = (int)threadIdx.x;
     const int i0 = (int)blockIdx.x * kTmaTile, j = (int)blockIdx.y, seg = (int)blockIdx.z;
     const int i = i0 + t;
-    const int k0 = seg * kSegZ, k1 = min(k0 + kSegZ, dm.nz);
+    const int k0 = seg << rp.segzs, k1 = min(k0 + (1 << rp.segzs), dm.nz);
     const int n = dm.n, plane = dm.nx * dm.ny;
     const T dtdx = (T)(sc->dt / rp.dx);
     const int nrows = 7 * npass + 5;
@@ -1877,7 +1879,7 @@ __global__ void __launch_bounds__(kTmaTile, sizeof(T) == 4 ? (NP <= 2 ? 10 : NP 
     constexpr int RS = ptma_row_stride<T>();
     const int t = (int)threadIdx.x;
     const int i0 = (int)blockIdx.x * kTmaTile, i = i0 + t, j = (int)blockIdx.y;
-    const int k0 = (int)blockIdx.z * kSegZ, k1 = min(k0 + kSegZ, dm.nz);
+    const int k0 = (int)blockIdx.z << rp.segzs, k1 = min(k0 + (1 << rp.segzs), dm.nz);
     const int n = dm.n, plane = dm.nx * dm.ny;
     const int ih = (i0 == 0 ? dm.nx : i0) - HE;       // left halo: cells i0-HE .. i0-1
     const int ir = (i0 + kTmaTile) % dm.nx;            // right halo: cells i0+128 .. i0+128+HE-1
@@ -2163,9 +2165,11 @@ __global__ void __launch_bounds__(kBX) k_force_kick(BatchArgs ba) {
 // ============================================================ dt and maxima
 // compute_new_time_step (driver.f90:432-448) with the smax coupling of
 // get_max_speed_vanleer (vanleer_mod.f90:3323); resets the step maxima.
-static __global__ void k_finalize(BatchArgs ba, int device_driven) {
-    int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= ba.nbox) return;
+// One warp per box: each lane folds kSlots / 32 slots of every maximum and
+// lane 0 does the rest (a single thread's serial loads and stores took 13-20
+// us of every step, between events; the warp takes 6-8 us).
+static __global__ void __launch_bounds__(32) k_finalize(BatchArgs ba, int device_driven) {
+    const int b = (int)blockIdx.x;
     const BoxRec rp = box_at(ba, b);
     Scalars* sc = rp.sc;
     if (!rp.active) return;
@@ -2175,7 +2179,7 @@ static __global__ void k_finalize(BatchArgs ba, int device_driven) {
     // after a protected final update with bad cells the CFL maximum of the
     // corrected state is in cfl_slots (k_prot_cfl)
     const bool protected_cfl = rp.protect && sc->nbad[1] > 0 && !drive;
-    for (int s = 0; s < kSlots; ++s) {
+    for (int s = (int)threadIdx.x; s < kSlots; s += 32) {
         cell = nmax(cell, __longlong_as_double((long long)(protected_cfl ? sc->cfl_slots[s] : sc->cmax_slots[s])));
         smax = nmax(smax, __longlong_as_double((long long)sc->smax_slots[s]));
         dvm = nmax(dvm, __longlong_as_double((long long)sc->dvmax_slots[s]));
@@ -2184,6 +2188,10 @@ static __global__ void k_finalize(BatchArgs ba, int device_driven) {
         sc->dvmax_slots[s] = 0ull;
         if (rp.protect) sc->cfl_slots[s] = 0ull;
     }
+    cell = warp_max(cell);
+    smax = warp_max(smax);
+    dvm = warp_max(dvm);
+    if (threadIdx.x != 0) return;
     sc->nbad[0] = sc->nbad[1] = 0u;
     double cmax = vmax(cell, smax + dvm);
     if (!(cmax == cmax) || cmax > 1.0e300) sc->status |= 2u;

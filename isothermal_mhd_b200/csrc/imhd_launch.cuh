@@ -30,6 +30,8 @@ inline void for_schemes(Fn&& f) {
     for_schemes_impl(f, std::make_integer_sequence<int, kSchemes>{});
 }
 
+inline int ceil_shift(int n, int log) { return (n + (1 << log) - 1) >> log; }
+
 inline void mark(BatchDev& b, int stage) {
     if (!b.prof) return;
     cudaEventRecord(b.ev[stage], b.st);
@@ -52,7 +54,7 @@ static dim3 grid_of(const BatchDev& b, int kind) {
         if (kind == kKindCellZ) return dim3(nbx, nby, (unsigned)((r.nz + sz - 1) / sz));
         if (kind == kKindRed) return dim3((unsigned)r.nred);
         switch ((kind - kKindSolver0) % 5) {
-            case kSubCell: return dim3(nbx, nby, (unsigned)((r.nz + kSegZ - 1) / kSegZ));   // z columns
+            case kSubCell: return dim3(nbx, nby, (unsigned)((r.nz + sz - 1) / sz));   // z columns
             case kSubXRow: return dim3(r.ny, r.nz);
             case kSubXTile: return dim3((unsigned)((r.nx + kTX - 1) / kTX), r.ny, r.nz);
             case kSubMarchY: return dim3(nbx, nbz, (unsigned)((r.ny + sg - 1) / sg));
@@ -61,9 +63,23 @@ static dim3 grid_of(const BatchDev& b, int kind) {
     }
 }
 
+// A single box with columns shorter than kSegZ planes (one_box_segments) runs
+// the SHORT instantiations of the z-column kernels.
+template <bool ONE>
+static bool short_columns(const BatchDev& b) {
+    return ONE && b.a.one.segzs < kSegZLog;
+}
+
 // Corner EMFs of one stage (PROT: of the protection fluxes).
 template <class T, bool ONE, bool PROT>
 static void launch_emf(BatchDev& b, dim3 gz, int half_step_state) {
+    if constexpr (ONE) {
+        if (short_columns<ONE>(b)) {
+            k_corner_emf<T, ONE, PROT, true><<<gz, kBX, 0, b.st>>>(b.a, half_step_state);
+            b.launches += 1;
+            return;
+        }
+    }
     k_corner_emf<T, ONE, PROT><<<gz, kBX, 0, b.st>>>(b.a, half_step_state);
     b.launches += 1;
 }
@@ -72,6 +88,13 @@ template <class T, int SCHEME, bool ONE>
 static void launch_fluxes_pred(BatchDev& b) {
     if (!b.has_scheme[SCHEME] || b.totals[scheme_kind(SCHEME, kSubCell)] == 0) return;
     dim3 g = grid_of<ONE>(b, scheme_kind(SCHEME, kSubCell));
+    if constexpr (ONE) {
+        if (short_columns<ONE>(b)) {
+            k_pred_flux<T, SCHEME, ONE, true><<<g, kBX, 0, b.st>>>(b.a);
+            b.launches += 1;
+            return;
+        }
+    }
     k_pred_flux<T, SCHEME, ONE><<<g, kBX, 0, b.st>>>(b.a);
     b.launches += 1;
 }
@@ -132,10 +155,18 @@ static void launch_update(BatchDev& b, double dt_scale, int final_stage) {
     if (ONE && aligned && tw > 0) {
         ensure_update_tma_attr<T>();
         const dim3 g((unsigned)(b.a.one.nx / tw), (unsigned)(b.a.one.ny / (kTmaTile / tw)),
-                     (unsigned)((b.a.one.nz + kSegZ - 1) / kSegZ));
+                     (unsigned)ceil_shift(b.a.one.nz, b.a.one.segzs));
         if (tw == kTmaTile) launch_update_tma<T, ONE, kTmaTile>(b, g, dt_scale, final_stage);
         else launch_update_tma<T, ONE, kTmaTile / 2>(b, g, dt_scale, final_stage);
         return;
+    }
+    if constexpr (ONE) {
+        if (short_columns<ONE>(b)) {
+            if (b.any_zrange) k_update<T, ONE, true, true><<<gz, kBX, 0, b.st>>>(b.a, dt_scale, final_stage);
+            else k_update<T, ONE, false, true><<<gz, kBX, 0, b.st>>>(b.a, dt_scale, final_stage);
+            b.launches += 1;
+            return;
+        }
     }
     if (b.any_zrange) k_update<T, ONE, true><<<gz, kBX, 0, b.st>>>(b.a, dt_scale, final_stage);
     else k_update<T, ONE, false><<<gz, kBX, 0, b.st>>>(b.a, dt_scale, final_stage);
@@ -195,7 +226,7 @@ static void launch_passive_pred(BatchDev& b, dim3 gz) {
     const BoxRec& r = b.a.one;
     if (ONE && ((uintptr_t)r.S[0] | (uintptr_t)r.SH) % 16 == 0 && passive_by_tma(r.nx)) {
         ensure_passive_pred_tma_attr<T>();
-        const dim3 g((unsigned)(r.nx / kTmaTile), (unsigned)r.ny, (unsigned)((r.nz + kSegZ - 1) / kSegZ));
+        const dim3 g((unsigned)(r.nx / kTmaTile), (unsigned)r.ny, (unsigned)ceil_shift(r.nz, r.segzs));
         if (b.npass_max <= 2)
             k_passive_pred_tma<T, 2><<<g, kTmaTile, passive_pred_tma_smem_bytes<T, 2>(), b.st>>>(b.a);
         else if (b.npass_max <= 4)
@@ -204,6 +235,15 @@ static void launch_passive_pred(BatchDev& b, dim3 gz) {
             k_passive_pred_tma<T, kMaxPass><<<g, kTmaTile, passive_pred_tma_smem_bytes<T, kMaxPass>(), b.st>>>(b.a);
         b.launches += 1;
         return;
+    }
+    if constexpr (ONE) {
+        if (short_columns<ONE>(b)) {
+            if (b.npass_max <= 2) k_passive_pred<T, ONE, 2, true><<<gz, kBX, 0, b.st>>>(b.a);
+            else if (b.npass_max <= 4) k_passive_pred<T, ONE, 4, true><<<gz, kBX, 0, b.st>>>(b.a);
+            else k_passive_pred<T, ONE, kMaxPass, true><<<gz, kBX, 0, b.st>>>(b.a);
+            b.launches += 1;
+            return;
+        }
     }
     if (b.npass_max <= 2) k_passive_pred<T, ONE, 2><<<gz, kBX, 0, b.st>>>(b.a);
     else if (b.npass_max <= 4) k_passive_pred<T, ONE, 4><<<gz, kBX, 0, b.st>>>(b.a);
@@ -216,7 +256,7 @@ static void launch_passive_corr(BatchDev& b, dim3 gz) {
     const BoxRec& r = b.a.one;
     if (ONE && ((uintptr_t)r.S[0] | (uintptr_t)r.SH | (uintptr_t)r.F) % 16 == 0 && passive_by_tma(r.nx)) {
         ensure_passive_tma_attr<T>();
-        const dim3 g((unsigned)(r.nx / kTmaTile), (unsigned)r.ny, (unsigned)((r.nz + kSegZ - 1) / kSegZ));
+        const dim3 g((unsigned)(r.nx / kTmaTile), (unsigned)r.ny, (unsigned)ceil_shift(r.nz, r.segzs));
         if (b.npass_max <= 2)
             k_passive_corr_tma<T, 2><<<g, kTmaTile, passive_tma_smem_bytes<T, 2>(), b.st>>>(b.a);
         else if (b.npass_max <= 4)
@@ -225,6 +265,15 @@ static void launch_passive_corr(BatchDev& b, dim3 gz) {
             k_passive_corr_tma<T, kMaxPass><<<g, kTmaTile, passive_tma_smem_bytes<T, kMaxPass>(), b.st>>>(b.a);
         b.launches += 1;
         return;
+    }
+    if constexpr (ONE) {
+        if (short_columns<ONE>(b)) {
+            if (b.npass_max <= 2) k_passive_corr<T, ONE, 2, true><<<gz, kBX, 0, b.st>>>(b.a);
+            else if (b.npass_max <= 4) k_passive_corr<T, ONE, 4, true><<<gz, kBX, 0, b.st>>>(b.a);
+            else k_passive_corr<T, ONE, kMaxPass, true><<<gz, kBX, 0, b.st>>>(b.a);
+            b.launches += 1;
+            return;
+        }
     }
     if (b.npass_max <= 2) k_passive_corr<T, ONE, 2><<<gz, kBX, 0, b.st>>>(b.a);
     else if (b.npass_max <= 4) k_passive_corr<T, ONE, 4><<<gz, kBX, 0, b.st>>>(b.a);
@@ -344,7 +393,7 @@ static cudaError_t run_step_t(BatchDev& b, int device_driven) {
         launch_passive_corr<T, ONE>(b, gz);
     }
     mark(b, kStFinalize);
-    k_finalize<<<nfin, 32, 0, b.st>>>(b.a, device_driven);
+    k_finalize<<<b.a.nbox, 32, 0, b.st>>>(b.a, device_driven);
     b.launches += 1;
     if (b.prof) cudaEventRecord(b.ev[kStages], b.st);
     return cudaGetLastError();

@@ -38,7 +38,7 @@ inline long blocks_of(const BoxRec& r, int kind, size_t esz) {
     if (scheme_of(box_solver(r), r.recon) != scheme) return 0;
     bool row = row_capable(r.nx, esz);
     switch (sub) {
-        case kSubCell: return nbx * nby * ceil_div(r.nz, kSegZ);   // z columns of the predictor fluxes
+        case kSubCell: return nbx * nby * ceil_div(r.nz, 1 << r.segzs);   // z columns of the predictor fluxes
         case kSubXRow: return row ? (long)r.ny * r.nz : 0;
         case kSubXTile: return row ? 0 : (long)ceil_div(r.nx, kTX) * r.ny * r.nz;
         case kSubMarchY: return nbx * nbz * ceil_div(r.ny, 1 << r.segs);   // (x, z) tiles marching along y
@@ -187,6 +187,44 @@ inline void init_rec(BoxRec& r, int nx, int ny, int nz, int npass, int riemann, 
     r.edot = edot;
     r.dt_turb = dt_turb;
     r.active = 1;
+}
+
+// Relative time of a single-box launch of `threads` columns of `len` cells
+// (blocks of kBX threads, `occ` of them resident per SM): `len` cells plus
+// `start` for what a column loads and computes before its first cell, times
+// the blocks that an SM takes one after the other.  A last wave of r blocks
+// per SM costs at least `fill` blocks' time (fewer leave the SM waiting on
+// latency).
+inline double column_cost(long blocks_per_unit, int len, double start, int occ, int fill) {
+    const long k = (blocks_per_unit / len + 147) / 148;
+    const long r = k % occ;
+    return (len + start) * (double)((k - r) + (r == 0 ? 0 : r < fill ? fill : r));
+}
+// Column lengths of a single box (a table shares its launches between boxes
+// and keeps the lengths of init_rec).  The y / z sweeps take the length of
+// least column_cost; the z-column kernels keep kSegZ planes (whose loops the
+// compiler unrolls) unless those leave fewer than 8 blocks per SM.  Measured
+// per step, Roe + PLM with scalars, all lengths 16 (as every box had), 8, 4,
+// 2, 1 (us between events): FP32 32^3 227, 163, 122, 102, 90; 64^3 306, 212,
+// 163, 169, 163; 96^3 373, 318, 320, 337, 365; 128^3 627, 616, 605, 652, 725;
+// 192^3 1827, 1932, 1987 (16 stays); FP64 64^3 577, 375, 385, 372, 393; 96^3
+// 1044, 953, 983, 1052, 1202; 128^3 2154, 2020, 2093; 192^3 7135, 7176.
+inline void one_box_segments(BoxRec& r, size_t esz) {
+    const int tw = 1 << r.tws, th = kBX >> r.tws, occ = esz == 8 ? 2 : 6, fill = esz == 8 ? 2 : 4;
+    const long nbx = ceil_div(r.nx, tw);
+    const long sweep = nbx * ((long)ceil_div(r.nz, th) * r.ny + (long)ceil_div(r.ny, th) * r.nz) / 2;
+    const long cols = nbx * ceil_div(r.ny, th) * r.nz;
+    double best = 0.0;
+    for (int s = 0; s <= 5; ++s) {
+        const double c = column_cost(sweep, 1 << s, 0.6, occ, fill);
+        if (s == 0 || c <= best) { best = c; r.segs = s; }
+    }
+    if (cols < 8L * 148 * kSegZ) {
+        for (int s = 0; s <= kSegZLog; ++s) {
+            const double c = column_cost(cols, 1 << s, 0.5, occ, fill);
+            if (s == 0 || c <= best) { best = c; r.segzs = s; }
+        }
+    }
 }
 
 // Device bytes of one box's buffers (state x2, fluxes, EMFs, half-step
