@@ -35,7 +35,7 @@ UNITS = {
     "imhd_server.cu": [],
     "imhd_io.cu": [],
 }
-HEADERS = ["imhd_physics.cuh", "imhd_physics_fast.cuh", "imhd_types.cuh", "imhd_table.h", "imhd_kernels.cuh", "imhd_launch.cuh"]
+HEADERS = ["imhd_physics.cuh", "imhd_physics_fast.cuh", "imhd_physics_table.cuh", "imhd_value.cuh", "imhd_types.cuh", "imhd_table.h", "imhd_kernels.cuh", "imhd_launch.cuh"]
 
 
 def nvcc() -> str:

@@ -155,7 +155,7 @@ imhd::BatchDev one_box(const imhd_batch* x, int box, int cur) {
     d.a.one.S[1] = r.S[cur ^ 1];
     d.a.one.active = 1;
     d.a.nbox = 1;
-    for (int k = 0; k < imhd::kKinds; ++k) d.totals[k] = (int)imhd::blocks_of(r, k, x->esz);
+    for (int k = 0; k < imhd::kKinds; ++k) d.totals[k] = (int)imhd::blocks_of(r, k, x->esz, x->b.row_pairs, true);
     d.prof = false;
     d.launches = 0;
     return d;
@@ -374,6 +374,7 @@ int apply_setting(imhd_batch* x, int tile, int segs, int segzs) {
     BCK(cudaStreamSynchronize(x->st));
     for (imhd::BoxRec& r : recs) {
         r.tws = tile_of(tile, r.nx);
+        r.ptws = (short)imhd::pair_tile(r.nx, r.tws);
         r.segs = segs;
         r.segzs = segzs;
     }

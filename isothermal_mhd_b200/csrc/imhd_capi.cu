@@ -88,7 +88,7 @@ void* cur_state(imhd_box* x) { return x->rec.S[x->cur]; }
 int upload_table(imhd_box* x) {
     std::vector<imhd::BoxRec> recs(1, x->rec);
     std::vector<int> prefix;
-    if (!imhd::build_prefix(recs, x->esz, prefix, x->b)) return fail(IMHD_E_ARG, "box too large for one launch");
+    if (!imhd::build_prefix(recs, x->esz, prefix, x->b, true)) return fail(IMHD_E_ARG, "box too large for one launch");
     CK(cudaMemcpyAsync(x->table, &x->rec, sizeof(imhd::BoxRec), cudaMemcpyHostToDevice, x->b.st));
     CK(cudaMemcpyAsync((char*)x->table + imhd::align256(sizeof(imhd::BoxRec)), prefix.data(), prefix.size() * sizeof(int),
                        cudaMemcpyHostToDevice, x->b.st));

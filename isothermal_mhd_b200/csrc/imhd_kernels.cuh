@@ -25,7 +25,10 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "imhd_physics_fast.cuh"
+#include "imhd_physics_table.cuh"
 #include "imhd_types.cuh"
 
 namespace imhd {
@@ -216,11 +219,10 @@ __device__ __forceinline__ void protection_flux(const T* uL, const T* uR, T cs, 
     }
 }
 
-// FP32 occupancy, measured at 512^3: five blocks per SM for the Roe solver
-// (96 registers; fewer registers spill more than the extra warps return), six
-// for HLLD and HLLE (80 registers, 3.9 -> 3.7 ms).
+// FP64, and FP32 Roe boxes of a table (five blocks per SM: 96 registers, fewer
+// spill more than the extra warps return); other FP32 boxes run k_pred_flux_f32.
 template <class T, int SCHEME, bool ONE, bool SHORT = false>
-__global__ void __launch_bounds__(kBX, sizeof(T) == 4 ? (scheme_solver(SCHEME) % 3 == 1 ? 5 : 6) : 1)
+__global__ void __launch_bounds__(kBX, sizeof(T) == 4 ? 5 : 1)
 k_pred_flux(BatchArgs ba) {
     constexpr int SOLVER = scheme_solver(SCHEME);
     int local;
@@ -321,9 +323,9 @@ __device__ __forceinline__ void store_flux(T* __restrict__ F, int D, int n, int 
 // marches along the sweep direction over a segment of faces.  PLM keeps the
 // primitive window w(a-1..a+2) and the slopes delw(a), delw(a+1) in
 // registers; PPM keeps w(a..a+3), the slopes delw(a), delw(a+1) and the right
-// edge of cell a.  Loads stay coalesced along x.
-// FP32: six blocks per SM (80 registers, a few spills): the z sweep had run
-// four blocks at 104 registers; 3.4 -> 3.1 ms (Roe, PLM) at 512^3.
+// edge of cell a.  Loads stay coalesced along x.  FP64, and FP32 Roe boxes of a
+// table (six blocks per SM, 80 registers, a few spills); other FP32 boxes run
+// k_sweep_f32.
 template <class T, int SCHEME, int D, bool ONE>
 __global__ void __launch_bounds__(kBX, sizeof(T) == 4 ? 6 : 1) k_corr_flux_march(BatchArgs ba) {
     constexpr int SOLVER = scheme_solver(SCHEME);
@@ -525,14 +527,11 @@ __global__ void __launch_bounds__(TX) k_corr_flux_x(BatchArgs ba) {
 // wrap is an index wrap inside the row, so every cell's slope is computed
 // exactly once (the tiled kernel above recomputes slopes at tile edges and
 // stages a halo).  PPM evaluates the edges of cells i and i+1 per face.
-// Needs 13 * nx * sizeof(T) bytes of dynamic shared memory.
-// FP32: 128-thread blocks (smaller barrier groups, 27 KB of shared memory
-// each at nx = 512): 3.45 -> 3.22 ms (Roe, PLM) at 512^3 against four
-// 256-thread blocks.  A single box runs six per SM at 80 registers without
-// spills (3.22 -> 3.19 ms); a table keeps eight at 64 (six: batched workload
-// 4.67 -> 4.58e9 cell-updates/s).
+// Needs 13 * nx * sizeof(T) bytes of dynamic shared memory.  FP64, and FP32 Roe
+// boxes of a table (eight blocks per SM at 64 registers; six: batched workload
+// 4.67 -> 4.58e9 cell-updates/s); other FP32 boxes run k_xrow_f32.
 template <class T, int SCHEME, bool ONE>
-__global__ void __launch_bounds__(128, sizeof(T) == 4 ? (ONE ? 6 : 8) : 1) k_corr_flux_xrow(BatchArgs ba) {
+__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 8 : 1) k_corr_flux_xrow(BatchArgs ba) {
     constexpr int SOLVER = scheme_solver(SCHEME);
     constexpr int RECON = scheme_recon(SCHEME);
     constexpr bool PPM = (RECON & 1) != 0, PRIM = (RECON & 2) != 0;
@@ -614,6 +613,481 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? (ONE ? 6 : 8) : 1) k_cor
     block_atomic_max_any(smax_slots, (double)smax);
 }
 
+// ============================================================ FP32 flux sweeps
+// The FP32 sweeps work on two interfaces at once (F2): the predictor and the
+// y / z sweeps on cells x and x+1 of a row, the x sweep on rows y and y+1.
+// An odd last cell or row is paired with its periodic neighbour, whose result
+// is dropped.  They are bound by the FP32 pipe (59-64% of its cycles at three
+// blocks of 158-168 registers per SM, 50-57% of the issue slots), where the
+// one-interface kernels were bound by issue (81-87%): half the instructions
+// per cell (y sweep 652 -> 339).  512^3 Roe + PLM, ms: predictor 4.32 -> 3.67,
+// x 3.29 -> 2.48, y 3.01 -> 2.03, z 3.12 -> 2.04.  Four blocks per SM (128
+// registers) spill: y 2.51.
+//
+// Lane offsets of a pair of cells: c0 and c1 = the next cell of the row.  vec:
+// the row length is even, so that c0 is even and both lanes are one aligned
+// 8-byte access.  No kernel writes what it reads this way, so the loads are
+// read-only ones, which may move above the stores of the face before.
+template <class V, bool VEC>
+__device__ __forceinline__ V ld_lanes(const float* __restrict__ p, int c0, int c1) {
+    if constexpr (lanes_of<V>::n == 1) {
+        return F1{__ldg(p + c0)};
+    } else if constexpr (VEC) {
+        return F2{__ldg((const unsigned long long*)(p + c0))};
+    } else {
+        return pack2(__ldg(p + c0), __ldg(p + c1));
+    }
+}
+// NF fields of S, f[0..NF-1], of a pair of cells
+template <bool VEC, class V, int NF>
+__device__ __forceinline__ void ld_fields(const float* __restrict__ S, int n, const int (&f)[NF], int c0, int c1, V* o) {
+#pragma unroll
+    for (int m = 0; m < NF; ++m) o[m] = ld_lanes<V, VEC>(S + (size_t)f[m] * n, c0, c1);
+}
+// The same with the row alignment tested at run time: one uniform branch
+// around all the loads.  In the sweeps it also keeps the loads of the next
+// cell where they are written, ahead of this face's arithmetic (without it
+// the compiler sinks them to their use: y sweep 2.03 -> 2.48 ms at 512^3).
+template <class V, int NF>
+__device__ __forceinline__ void ld_fields_any(const float* __restrict__ S, int n, const int (&f)[NF], int c0, int c1,
+                                              bool vec, V* o) {
+    if (lanes_of<V>::n == 1 || vec) ld_fields<true>(S, n, f, c0, c1, o);
+    else ld_fields<false>(S, n, f, c0, c1, o);
+}
+// the six flux components of sweep D (two: the second lane's cell is its own)
+template <bool VEC, class V>
+__device__ __forceinline__ void st_flux(float* __restrict__ F, int D, int n, int c0, int c1, bool two, const V* Fo) {
+    float* Fd = F + (size_t)(6 * D) * n;
+    if constexpr (lanes_of<V>::n == 1) {
+#pragma unroll
+        for (int m = 0; m < 6; ++m) Fd[(size_t)m * n + c0] = Fo[m].v;
+    } else if constexpr (VEC) {
+#pragma unroll
+        for (int m = 0; m < 6; ++m) *(unsigned long long*)(Fd + (size_t)m * n + c0) = Fo[m].v;
+    } else {
+#pragma unroll
+        for (int m = 0; m < 6; ++m) {
+            float a, b;
+            unpack2(Fo[m], a, b);
+            Fd[(size_t)m * n + c0] = a;
+            if (two) Fd[(size_t)m * n + c1] = b;
+        }
+    }
+}
+template <class V>
+__device__ __forceinline__ void st_flux_any(float* __restrict__ F, int D, int n, int c0, int c1, bool vec, bool two,
+                                            const V* Fo) {
+    if (lanes_of<V>::n == 2 && vec) st_flux<true>(F, D, n, c0, c1, two, Fo);
+    else st_flux<false>(F, D, n, c0, c1, two, Fo);
+}
+// flux of a face, and the protection (HLLE) flux beside it for solver 4
+template <int SOLVER, class V>
+__device__ __forceinline__ void face_fast(const Side<V>& L, const Side<V>& R, V bn, float cs, float asqr, V& smax,
+                                          const BoxRec& rp, int D, int c0, int c1, bool vec, bool two) {
+    V Fo[6];
+    riemann_fast<SOLVER>(L, R, bn, cs, asqr, Fo, smax);
+    st_flux_any((float*)rp.F, D, rp.n, c0, c1, vec, two, Fo);
+    if constexpr (SOLVER == 4) {
+        flux_hlle_fast(L, R, bn, asqr, Fo, smax);
+        st_flux_any((float*)rp.Fp, D, rp.n, c0, c1, vec, two, Fo);
+    }
+}
+
+// Predictor fluxes (k_pred_flux) of the faces x+1/2, y+1/2, z+1/2 of a pair of
+// cells, marching along z: the state and velocity of the plane above are
+// those of the next plane, the x neighbour of the first cell is the second
+// one.
+struct CellF2 {
+    F2 r, m[3], v[3], b[3], bf[3];
+};
+template <int A, int B, int C>
+__device__ __forceinline__ void cell_side(const CellF2& a, Side<F2>& s) {
+    s.r = a.r;
+    s.v[0] = a.v[A]; s.v[1] = a.v[B]; s.v[2] = a.v[C];
+    s.m[0] = a.m[A]; s.m[1] = a.m[B]; s.m[2] = a.m[C];
+    s.b[0] = a.b[B]; s.b[1] = a.b[C];
+}
+__device__ __forceinline__ void to_cell(const F2* u, CellF2& a) {
+    const F2 ir = vrcp(u[0]);
+    a.r = u[0];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        a.m[d] = u[1 + d];
+        a.v[d] = u[1 + d] * ir;
+        a.b[d] = u[4 + d];
+        a.bf[d] = u[7 + d];
+    }
+}
+template <int SOLVER, bool ONE>
+__device__ __forceinline__ void pred_flux_f32(const BoxRec& rp, int local, bool vec) {
+    const Dims dm = dims_of(rp);
+    const float* __restrict__ S = (const float*)rp.S[0];
+    const float cs = (float)rp.cs, asqr = (float)(rp.cs * rp.cs);
+    int p, j, k0, k1;
+    decode_cellz<ONE, true>(local, Dims{(dm.nx + 1) / 2, dm.ny, dm.nz, 0}, rp.ptws, rp.segzs, p, j, k0, k1);
+    F2 smax = same<F2>(0.0f);
+    if (2 * p < dm.nx && j < dm.ny) {
+        const int n = dm.n, plane = dm.nx * dm.ny;
+        const int x0 = 2 * p, x1 = wrap_up(x0, dm.nx), x2 = wrap_up(x1, dm.nx);
+        const bool two = x0 + 1 < dm.nx;
+        const int row = dm.nx * j, rowp = dm.nx * wrap_up(j, dm.ny);
+        const int all[10] = {0, 1, 2, 3, 4, 5, 6, 7, 8, 9};
+        CellF2 cur;
+        {
+            F2 u[10];
+            ld_fields_any(S, n, all, row + x0 + k0 * plane, row + x1 + k0 * plane, vec, u);
+            to_cell(u, cur);
+        }
+        for (int k = k0; k < k1; ++k) {
+            const int kp = k * plane, kz = wrap_up(k, dm.nz) * plane, c0 = row + x0 + kp, c1 = row + x1 + kp;
+            F2 sdrop = smax;     // faces outside zlo..zhi-1 do not enter smax
+            F2& sref = (k >= rp.zlo && k < rp.zhi) ? smax : sdrop;
+            // this plane's y row and the plane above, loaded before the x face
+            float e[6];
+            F2 u[6], z[10];
+            {
+                const int f[6] = {0, 1, 2, 3, 5, 6}, fy[6] = {0, 1, 2, 3, 4, 6};
+#pragma unroll
+                for (int m = 0; m < 6; ++m) e[m] = __ldg(fld(S, f[m], n) + (row + x2 + kp));
+                if (vec) {
+                    ld_fields<true>(S, n, fy, rowp + x0 + kp, rowp + x1 + kp, u);
+                    ld_fields<true>(S, n, all, row + x0 + kz, row + x1 + kz, z);
+                } else {
+                    ld_fields<false>(S, n, fy, rowp + x0 + kp, rowp + x1 + kp, u);
+                    ld_fields<false>(S, n, all, row + x0 + kz, row + x1 + kz, z);
+                }
+            }
+            CellF2 up;
+            Side<F2> L, R;
+            {
+                const float ir = 1.0f / e[0];
+                auto next = [](F2 a, float b) { float x, y; unpack2(a, x, y); return pack2(y, b); };
+                R.r = next(cur.r, e[0]);
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    R.m[d] = next(cur.m[d], e[1 + d]);
+                    R.v[d] = next(cur.v[d], __fmul_rn(e[1 + d], ir));
+                }
+                R.b[0] = next(cur.b[1], e[4]);
+                R.b[1] = next(cur.b[2], e[5]);
+                cell_side<0, 1, 2>(cur, L);
+                face_fast<SOLVER>(L, R, cur.bf[0], cs, asqr, sref, rp, 0, c0, c1, vec, two);
+            }
+            {
+                const F2 ir = vrcp(u[0]);
+                R.r = u[0];
+                R.m[0] = u[2]; R.m[1] = u[3]; R.m[2] = u[1];
+#pragma unroll
+                for (int d = 0; d < 3; ++d) R.v[d] = R.m[d] * ir;
+                R.b[0] = u[5]; R.b[1] = u[4];
+                cell_side<1, 2, 0>(cur, L);
+                face_fast<SOLVER>(L, R, cur.bf[1], cs, asqr, sref, rp, 1, c0, c1, vec, two);
+            }
+            to_cell(z, up);
+            cell_side<2, 0, 1>(cur, L);
+            cell_side<2, 0, 1>(up, R);
+            face_fast<SOLVER>(L, R, cur.bf[2], cs, asqr, sref, rp, 2, c0, c1, vec, two);
+            cur = up;
+        }
+    }
+    block_atomic_max<kBX>(rp.sc->smax_slots, (double)top_lane(smax));
+}
+// Roe: one body per row alignment, which the compiler schedules better (438
+// against 479 us at 256^3); HLLD and HLLE: one body that tests it at each
+// group of loads (492 against 530 us).
+template <int SOLVER, bool ONE>
+__global__ void __launch_bounds__(kBX, 3) k_pred_flux_f32(BatchArgs ba, int kind) {
+    int local;
+    const BoxRec rp = resolve<ONE>(ba, kind, local);
+    if (!rp.active) return;
+    if constexpr (SOLVER == 1 || SOLVER == 4) {
+        if (rp.vec) pred_flux_f32<SOLVER, ONE>(rp, local, true);
+        else pred_flux_f32<SOLVER, ONE>(rp, local, false);
+    } else {
+        pred_flux_f32<SOLVER, ONE>(rp, local, rp.vec != 0);
+    }
+}
+
+// Primitives (rho, v_n, v_t1, v_t2, B_t1, B_t2) and normal face field of
+// sweep D from the seven loaded fields (load_prim).
+template <class V, int D>
+__device__ __forceinline__ void ld_raw(const float* __restrict__ S, int n, int c0, int c1, bool vec, V* u) {
+    using R = Rot<D>;
+    const int f[7] = {0, R::MN, R::MT1, R::MT2, R::BT1, R::BT2, R::BN};
+    ld_fields_any(S, n, f, c0, c1, vec, u);
+}
+template <class V>
+__device__ __forceinline__ void to_prim(const V* u, V* w, V& bn) {
+    const V ir = vrcp(u[0]);
+    w[0] = u[0];
+#pragma unroll
+    for (int m = 1; m < 4; ++m) w[m] = u[m] * ir;
+    w[4] = u[4];
+    w[5] = u[5];
+    bn = u[6];
+}
+
+template <class V, int D>
+__device__ __forceinline__ void ld_prim(const float* __restrict__ S, int n, int c0, int c1, bool vec, V* w, V& bn) {
+    V u[7];
+    ld_raw<V, D>(S, n, c0, c1, vec, u);
+    to_prim(u, w, bn);
+}
+
+// Corrector sweeps along y and z (k_corr_flux_march); PPM works on one cell
+// per thread, whose larger window would not fit two.
+template <int SCHEME, int D, bool ONE>
+__global__ void __launch_bounds__(kBX, (scheme_recon(SCHEME) & 1) ? 6 : 3) k_sweep_f32(BatchArgs ba) {
+    int local;
+    const BoxRec rp = resolve<ONE>(ba, scheme_kind(SCHEME, D == 1 ? kSubMarchY : kSubMarchZ), local);
+    if (!rp.active) return;
+    const bool vec = rp.vec != 0;
+    constexpr int SOLVER = scheme_solver(SCHEME);
+    constexpr int RECON = scheme_recon(SCHEME);
+    constexpr bool PPM = (RECON & 1) != 0, PRIM = (RECON & 2) != 0;
+    using V = std::conditional_t<PPM, F1, F2>;
+    constexpr int W = lanes_of<V>::n;
+    const Dims dm = dims_of(rp);
+    const float* __restrict__ S = (const float*)rp.S[1];   // half-step state
+    const float cs = (float)rp.cs, asqr = (float)(rp.cs * rp.cs);
+    const int seg = 1 << rp.segs, tws = PPM ? rp.tws : rp.ptws;
+    const int nother = (D == 1) ? dm.nz : dm.ny, nunits = (dm.nx + W - 1) / W;
+    const int tw = 1 << tws, th = kBX >> tws;
+    int bx, bo, a0;
+    if constexpr (ONE) {                        // grid (nbx, nbo, nseg)
+        bx = (int)blockIdx.x; bo = (int)blockIdx.y; a0 = (int)blockIdx.z * seg;
+    } else {
+        int nbx = (nunits + tw - 1) >> tws, nbo = (nother + th - 1) / th;
+        int rest = local / nbx;
+        bx = local % nbx;
+        bo = rest % nbo;
+        a0 = (rest / nbo) * seg;
+    }
+    const int x0 = W * (bx * tw + ((int)threadIdx.x & (tw - 1)));
+    const int o = bo * th + ((int)threadIdx.x >> tws);   // k for D=1, j for D=2
+    const int na = (D == 1) ? dm.ny : dm.nz;
+    const int a1 = min(a0 + seg, na);
+    V smax = same<V>(0.0f);
+    if (x0 < dm.nx && o < nother) {
+        const int n = dm.n, stride = (D == 1) ? dm.nx : dm.nx * dm.ny;
+        const int base0 = x0 + ((D == 1) ? dm.nx * dm.ny * o : dm.nx * o);
+        const int base1 = base0 + (wrap_up(x0, dm.nx) - x0);
+        const bool two = x0 + 1 < dm.nx;
+        auto prim = [&](int a, V* w, V& bn) { ld_prim<V, D>(S, n, base0 + a * stride, base1 + a * stride, vec, w, bn); };
+        if constexpr (!PPM) {
+            V wb_[6], wc[6], wd[6];          // w(a), w(a+1), w(a+2)
+            V bnA, bnB, bnC;
+            V dA[6], dB[6];                  // delw(a), delw(a+1)
+            prim(wrap_any(a0 - 1, na), wd, bnC);
+            prim(a0, wb_, bnA);
+            prim(wrap_up(a0, na), wc, bnB);
+            recon_slope_fast<RECON>(wd, wb_, wc, wc, bnA, cs, asqr, dA);
+            V raw[7];                        // fields of cell a+2, loaded one face ahead
+            int ar = wrap_up(wrap_up(a0, na), na);
+            ld_raw<V, D>(S, n, base0 + ar * stride, base1 + ar * stride, vec, raw);
+#pragma unroll 1
+            for (int a = a0; a < a1; ++a) {
+                to_prim(raw, wd, bnC);
+                ar = wrap_up(ar, na);
+                ld_raw<V, D>(S, n, base0 + ar * stride, base1 + ar * stride, vec, raw);
+                recon_slope_fast<RECON>(wb_, wc, wd, wd, bnB, cs, asqr, dB);
+                Side<V> L, R;
+                plm_side(wb_, dA, 0.5f, L);
+                plm_side(wc, dB, -0.5f, R);
+                const int kf = (D == 1) ? o : a;
+                V sdrop = smax;
+                V& sref = (kf >= rp.zlo && kf < rp.zhi) ? smax : sdrop;
+                face_fast<SOLVER>(L, R, bnA, cs, asqr, sref, rp, D, base0 + a * stride, base1 + a * stride, vec, two);
+#pragma unroll
+                for (int m = 0; m < 6; ++m) { wb_[m] = wc[m]; wc[m] = wd[m]; dA[m] = dB[m]; }
+                bnA = bnB; bnB = bnC;
+            }
+        } else {
+            V w0[6], w1[6], w2[6], w3[6];    // w(a), w(a+1), w(a+2), w(a+3)
+            V bn0, bn1, bn2, bn3;
+            V d0[6], d1[6];                  // delw(a), delw(a+1)
+            V r0[6];                         // right edge of cell a
+            {
+                V wm2[6], wm1[6], dm1[6], l0[6], bnm2, bnm1;
+                prim(wrap_any(a0 - 2, na), wm2, bnm2);
+                prim(wrap_any(a0 - 1, na), wm1, bnm1);
+                prim(a0, w0, bn0);
+                prim(wrap_any(a0 + 1, na), w1, bn1);
+                prim(wrap_any(a0 + 2, na), w2, bn2);
+                recon_slope_fast<RECON>(wm2, wm1, w0, w1, bnm1, cs, asqr, dm1);
+                recon_slope_fast<RECON>(wm1, w0, w1, w2, bn0, cs, asqr, d0);
+                ppm_edges_fast<PRIM>(wm1, w0, w1, dm1, d0, l0, r0);
+            }
+#pragma unroll 1
+            for (int a = a0; a < a1; ++a) {
+                prim(wrap_any(a + 3, na), w3, bn3);
+                recon_slope_fast<RECON>(w0, w1, w2, w3, bn1, cs, asqr, d1);
+                V l1[6], r1[6];
+                ppm_edges_fast<PRIM>(w0, w1, w2, d0, d1, l1, r1);
+                Side<V> L, R;
+                side_of(r0, L);
+                side_of(l1, R);
+                const int kf = (D == 1) ? o : a;
+                V sdrop = smax;
+                V& sref = (kf >= rp.zlo && kf < rp.zhi) ? smax : sdrop;
+                face_fast<SOLVER>(L, R, bn0, cs, asqr, sref, rp, D, base0 + a * stride, base1 + a * stride, vec, two);
+#pragma unroll
+                for (int m = 0; m < 6; ++m) {
+                    w0[m] = w1[m]; w1[m] = w2[m]; w2[m] = w3[m];
+                    d0[m] = d1[m]; r0[m] = r1[m];
+                }
+                bn0 = bn1; bn1 = bn2; bn2 = bn3;
+            }
+        }
+    }
+    block_atomic_max<kBX>(rp.sc->smax_slots, (double)top_lane(smax));
+}
+
+// Flux of the face right of staged cell q (row stride ST, cells q-1 .. q+2 at
+// the given staged positions) from the staged primitives and slopes.
+template <int SCHEME, class V>
+__device__ __forceinline__ void row_face(const V* sw, const V* sd, int ws, int ds, int qm, int q, int qp, int qp2, int um,
+                                         int u, int up, V bn, float cs, float asqr, V& sref, const BoxRec& rp, int c0,
+                                         int c1, bool two) {
+    constexpr int SOLVER = scheme_solver(SCHEME);
+    constexpr bool PPM = (scheme_recon(SCHEME) & 1) != 0, PRIM = (scheme_recon(SCHEME) & 2) != 0;
+    Side<V> L, R;
+    V w0[6], wp[6], d0[6], dp[6];
+#pragma unroll
+    for (int m = 0; m < 6; ++m) {
+        w0[m] = sw[m * ws + q]; wp[m] = sw[m * ws + qp];
+        d0[m] = sd[m * ds + u]; dp[m] = sd[m * ds + up];
+    }
+    if constexpr (!PPM) {
+        plm_side(w0, d0, 0.5f, L);
+        plm_side(wp, dp, -0.5f, R);
+    } else {
+        V wm[6], wp2[6], dm1[6], l[6], r[6], l1[6], r1[6];
+#pragma unroll
+        for (int m = 0; m < 6; ++m) { wm[m] = sw[m * ws + qm]; wp2[m] = sw[m * ws + qp2]; dm1[m] = sd[m * ds + um]; }
+        ppm_edges_fast<PRIM>(wm, w0, wp, dm1, d0, l, r);      // cell q
+        ppm_edges_fast<PRIM>(w0, wp, wp2, d0, dp, l1, r1);    // cell q+1
+        side_of(r, L);
+        side_of(l1, R);
+    }
+    face_fast<SOLVER>(L, R, bn, cs, asqr, sref, rp, 0, c0, c1, false, two);
+}
+
+// Sweep along x over whole rows (k_corr_flux_xrow): F2 blocks stage two rows
+// y, y+1 side by side.  13 * nx * sizeof(V) bytes of shared memory.
+template <int SCHEME, class V, bool ONE>
+__global__ void __launch_bounds__(128, lanes_of<V>::n == 2 ? (scheme_solver(SCHEME) % 3 == 1 ? 4 : 5) : 8) k_xrow_f32(BatchArgs ba) {
+    constexpr int RECON = scheme_recon(SCHEME), W = lanes_of<V>::n;
+    constexpr bool PPM = (RECON & 1) != 0;
+    extern __shared__ __align__(16) unsigned char xrow_smem[];
+    int local;
+    const BoxRec rp = resolve<ONE>(ba, scheme_kind(SCHEME, kSubXRow), local);
+    if (!rp.active) return;
+    const Dims dm = dims_of(rp);
+    const float* __restrict__ S = (const float*)rp.S[1];   // half-step state
+    const float cs = (float)rp.cs, asqr = (float)(rp.cs * rp.cs);
+    const int nx = dm.nx;
+    V* sw = (V*)xrow_smem;     // [6][nx] primitives
+    V* sbn = sw + 6 * nx;      // [nx] face field at i+1/2
+    V* sd = sbn + nx;          // [6][nx] slopes
+    int j, k;
+    if constexpr (ONE) {                        // grid (ceil(ny / W), nz)
+        j = (int)blockIdx.x * W; k = (int)blockIdx.y;
+    } else {
+        const int nyw = (dm.ny + W - 1) / W;
+        j = (local % nyw) * W; k = local / nyw;
+    }
+    const int row0 = nx * (j + dm.ny * k), row1 = nx * (wrap_up(j, dm.ny) + dm.ny * k);
+    const bool two = j + 1 < dm.ny;
+    for (int i = threadIdx.x; i < nx; i += blockDim.x) {
+        V w[6], bn;
+        ld_prim<V, 0>(S, dm.n, row0 + i, row1 + i, false, w, bn);
+#pragma unroll
+        for (int m = 0; m < 6; ++m) sw[m * nx + i] = w[m];
+        sbn[i] = bn;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < nx; i += blockDim.x) {
+        const int im = wrap_dn(i, nx), ip = wrap_up(i, nx), ip2 = wrap_up(ip, nx);
+        V wm[6], w0[6], wp[6], wp2[6], d[6];
+#pragma unroll
+        for (int m = 0; m < 6; ++m) {
+            wm[m] = sw[m * nx + im]; w0[m] = sw[m * nx + i]; wp[m] = sw[m * nx + ip];
+            wp2[m] = PPM ? sw[m * nx + ip2] : wp[m];
+        }
+        recon_slope_fast<RECON>(wm, w0, wp, wp2, sbn[i], cs, asqr, d);
+#pragma unroll
+        for (int m = 0; m < 6; ++m) sd[m * nx + i] = d[m];
+    }
+    __syncthreads();
+    V smax = same<V>(0.0f);
+    for (int i = threadIdx.x; i < nx; i += blockDim.x) {
+        const int im = wrap_dn(i, nx), ip = wrap_up(i, nx), ip2 = wrap_up(ip, nx);
+        V sdrop = smax;
+        V& sref = (k >= rp.zlo && k < rp.zhi) ? smax : sdrop;
+        row_face<SCHEME>(sw, sd, nx, nx, im, i, ip, ip2, im, i, ip, sbn[i], cs, asqr, sref, rp, row0 + i, row1 + i, two);
+    }
+    block_atomic_max_any(rp.sc->smax_slots, (double)top_lane(smax));
+}
+
+// Sweep along x on tiles of TX faces (k_corr_flux_x), for rows too long for
+// the whole-row kernel.
+template <int SCHEME, int TX, bool ONE>
+__global__ void __launch_bounds__(TX) k_xtile_f32(BatchArgs ba) {
+    constexpr int RECON = scheme_recon(SCHEME);
+    constexpr bool PPM = (RECON & 1) != 0;
+    constexpr int H = PPM ? 2 : 1;           // cells staged left of the tile
+    constexpr int NW = TX + (PPM ? 5 : 3);   // staged cells
+    constexpr int ND = TX + (PPM ? 2 : 1);   // staged slopes, cells i0-H+1 ...
+    __shared__ F1 sw[6 * NW], sbn[NW], sd[6 * ND];
+    int local;
+    const BoxRec rp = resolve<ONE>(ba, scheme_kind(SCHEME, kSubXTile), local);
+    if (!rp.active) return;
+    const Dims dm = dims_of(rp);
+    const float* __restrict__ S = (const float*)rp.S[1];   // half-step state
+    const float cs = (float)rp.cs, asqr = (float)(rp.cs * rp.cs);
+    int i0, j, k;
+    if constexpr (ONE) {                        // grid (nbt, ny, nz)
+        i0 = (int)blockIdx.x * TX; j = (int)blockIdx.y; k = (int)blockIdx.z;
+    } else {
+        int nbt = (dm.nx + TX - 1) / TX;
+        i0 = (local % nbt) * TX;
+        j = (local / nbt) % dm.ny;
+        k = (local / nbt) / dm.ny;
+    }
+    const int row = dm.nx * (j + dm.ny * k);
+    for (int t = threadIdx.x; t < NW; t += TX) {   // staged cell t is i0 - H + t
+        const int c = row + wrap_any(i0 - H + t, dm.nx);
+        F1 w[6], bn;
+        ld_prim<F1, 0>(S, dm.n, c, c, false, w, bn);
+#pragma unroll
+        for (int m = 0; m < 6; ++m) sw[m * NW + t] = w[m];
+        sbn[t] = bn;
+    }
+    __syncthreads();
+    for (int u = threadIdx.x; u < ND; u += TX) {   // slope u is that of staged cell u + 1
+        F1 wm[6], w0[6], wp[6], wp2[6], d[6];
+#pragma unroll
+        for (int m = 0; m < 6; ++m) {
+            wm[m] = sw[m * NW + u]; w0[m] = sw[m * NW + u + 1]; wp[m] = sw[m * NW + u + 2];
+            wp2[m] = sw[m * NW + u + (PPM ? 3 : 2)];
+        }
+        recon_slope_fast<RECON>(wm, w0, wp, wp2, sbn[u + 1], cs, asqr, d);
+#pragma unroll
+        for (int m = 0; m < 6; ++m) sd[m * ND + u] = d[m];
+    }
+    __syncthreads();
+    const int t = threadIdx.x, i = i0 + t;
+    F1 smax = same<F1>(0.0f);
+    if (i < dm.nx) {   // cell i is staged at t + H, its slope at t + H - 1
+        F1 sdrop = smax;
+        F1& sref = (k >= rp.zlo && k < rp.zhi) ? smax : sdrop;
+        row_face<SCHEME>(sw, sd, NW, ND, t + H - 1, t + H, t + H + 1, t + (PPM ? H + 2 : H + 1), t + (PPM ? H - 2 : H - 1),
+                         t + H - 1, t + H, sbn[t + H], cs, asqr, sref, rp, row + i, row + i, true);
+    }
+    block_atomic_max<TX>(rp.sc->smax_slots, (double)smax.v);
+}
+
 // ============================================================ corner EMF
 // compute_cell_center_emf_3d (vanleer_mod.f90:1823-1862) evaluated on the fly
 // and compute_cell_corner_emf_3d (:1884-2076).  Face EMFs come from the flux
@@ -672,12 +1146,9 @@ __device__ __forceinline__ CellEV<T> cell_ev(const T* __restrict__ S, int n, int
 // PROT: the corner EMFs of the protection fluxes (Fp -> Ep) of the boxes
 // that compute them, the second compute_cell_corner_emf_3d call of
 // vanleer_mod.f90:336, 396 (the cell-centre EMFs are the same).
-// FP32 occupancy: six blocks per SM for a single box (eight spilled more than
-// they gained, 2.2 -> 2.4 ms at 512^3); eight in a table, whose small boxes
-// leave the loads less overlapped (the batched workload 4.48 -> 4.70e9
-// cell-updates/s).
+// FP64; FP32 runs k_corner_emf_f32.
 template <class T, bool ONE, bool PROT = false, bool SHORT = false>
-__global__ void __launch_bounds__(kBX, sizeof(T) == 4 ? (ONE ? 6 : 8) : 1) k_corner_emf(BatchArgs ba,
+__global__ void __launch_bounds__(kBX, 1) k_corner_emf(BatchArgs ba,
                                                                                        int half_step_state) {
     int local;
     const BoxRec rp = resolve<ONE>(ba, kKindCellZ, local);
@@ -786,6 +1257,178 @@ __global__ void __launch_bounds__(kBX, sizeof(T) == 4 ? (ONE ? 6 : 8) : 1) k_cor
     }
 }
 
+// ------------------------------------------------------------ FP32 corner EMF
+// k_corner_emf on a pair of cells per thread: the second cell is the x
+// neighbour of the first, so a pair evaluates 2 + 1 cells of each of its two
+// rows per plane where two threads evaluated 6, every load of a row is 8
+// bytes.  The upwinded differences are selected after they are subtracted (both
+// halves take the same side); in a table the results are those of k_corner_emf
+// compiled for float, to the bit.  Bound
+// by memory latency and bandwidth: 2.24 -> 1.57 ms at 512^3, 5.5 TB/s of the
+// algorithmic 64 B per cell (70% of DRAM peak in ncu at 256^3), with one body
+// per row alignment so that a plane's loads leave together (a test at each
+// group of loads: 2.51 ms); three or five blocks per SM: 1.80, 1.76 ms.
+template <class V>
+struct CellE {
+    V ex, ey, ez, ux, uy, uz;    // cell-centre EMF (ecc3) and velocity
+};
+template <class V>
+__device__ __forceinline__ void cell_e(const V* u, CellE<V>& o) {
+    const V ir = vrcp(u[0]), neg = same<V>(-1.0f);
+    o.ux = u[1] * ir;
+    o.uy = u[2] * ir;
+    o.uz = u[3] * ir;
+    o.ex = fma(u[5], u[3], (neg * u[6]) * u[2]) * ir;
+    o.ey = fma(u[6], u[1], (neg * u[4]) * u[3]) * ir;
+    o.ez = fma(u[4], u[2], (neg * u[5]) * u[1]) * ir;
+}
+// the pair one cell to the right (e: the cell after the pair) or left (e: the cell before it)
+__device__ __forceinline__ F2 right_of(F2 a, F1 e) {
+    float x, y;
+    unpack2(a, x, y);
+    return pack2(y, e.v);
+}
+__device__ __forceinline__ F2 left_of(F2 a, F1 e) {
+    float x, y;
+    unpack2(a, x, y);
+    return pack2(e.v, x);
+}
+// The difference of the upwind values 14 and 34 (upwind_pair) with the velocity
+// sum s = 2 v: left where s > 0, right where s < 0, and (near only) the means
+// where it is 0.
+__device__ __forceinline__ F2 upwind_diff(F2 s, bool near, F2 L14, F2 L34, F2 R14, F2 R34) {
+    const F2 l = L14 - L34, r = R14 - R34;
+    F2 d = vsel(s, l, r);
+    if (near) {
+        const float z = (float)(2.0 * kZERO);
+        d = each([z](float v, float a, float h) { return v > z ? a : v < -z ? a : h; }, s, d,
+                 same<F2>(0.5f) * (L14 + R14) - same<F2>(0.5f) * (L34 + R34));
+    }
+    return d;
+}
+// Whether the sum of two velocities, formed as products, may differ in sign
+// from the sum of the quotients (tol > 0), or is 0 (tol = 0).
+__device__ __forceinline__ bool near_zero(F2 a, F2 b, float tol) {
+    float a0, a1, b0, b1;
+    unpack2(a, a0, a1);
+    unpack2(b, b0, b1);
+    const float z = (float)(2.0 * kZERO);
+    const float t0 = tol > 0.0f ? tol * (fabsf(a0) + fabsf(b0)) : z, t1 = tol > 0.0f ? tol * (fabsf(a1) + fabsf(b1)) : z;
+    return !(fabsf(a0 + b0) > t0) || !(fabsf(a1 + b1) > t1);
+}
+template <bool VEC>
+__device__ __forceinline__ void st_lanes(float* __restrict__ p, int c0, int c1, bool two, F2 a) {
+    if constexpr (VEC) {
+        *(unsigned long long*)(p + c0) = a.v;
+    } else {
+        float x, y;
+        unpack2(a, x, y);
+        p[c0] = x;
+        if (two) p[c1] = y;
+    }
+}
+template <bool ONE, bool PROT, bool VEC>
+__device__ __forceinline__ void do_corner_emf_f32(const BoxRec& rp, int local, int half_step_state) {
+    const Dims dm = dims_of(rp);
+    const float* __restrict__ S = (const float*)(half_step_state ? rp.S[1] : rp.S[0]);
+    const float* __restrict__ F = (const float*)(PROT ? rp.Fp : rp.F);
+    float* __restrict__ E = (float*)(PROT ? rp.Ep : rp.E);
+    int p, j, k0, k1;
+    decode_cellz<ONE, true>(local, Dims{pairs_of(dm.nx), dm.ny, dm.nz, 0}, rp.ptws, rp.segzs, p, j, k0, k1);
+    if (2 * p >= dm.nx || j >= dm.ny) return;
+    const int n = dm.n, plane = dm.nx * dm.ny;
+    const int x0 = 2 * p, x1 = wrap_up(x0, dm.nx), x2 = wrap_up(x1, dm.nx), row = dm.nx * j, rowp = dm.nx * wrap_up(j, dm.ny);
+    const bool two = x0 + 1 < dm.nx;
+    const int r0 = row + x0, r1 = row + x1, r2 = row + x2, q0 = rowp + x0, q1 = rowp + x1, q2 = rowp + x2;
+    // what a plane gives: the pair's cells, x+1 of them, row j+1, x+1 of it
+    struct Plane {
+        CellE<F2> a;
+        F2 xey, xez, xux, bex, bez, buy, bxez, fx2, fy1;
+    };
+    auto load = [&](int kp, Plane& o) {
+        const int all[7] = {0, 1, 2, 3, 4, 5, 6};
+        F2 u[7];
+        F1 e[7];
+        CellE<F1> ce;
+        CellE<F2> cb;
+        ld_fields<VEC>(S, n, all, r0 + kp, r1 + kp, u);
+        ld_fields<VEC>(S, n, all, r2 + kp, 0, e);
+        cell_e(u, o.a);
+        cell_e(e, ce);
+        o.xey = right_of(o.a.ey, ce.ey);
+        o.xez = right_of(o.a.ez, ce.ez);
+        o.xux = right_of(o.a.ux, ce.ux);
+        ld_fields<VEC>(S, n, all, q0 + kp, q1 + kp, u);
+        ld_fields<VEC>(S, n, all, q2 + kp, 0, e);
+        cell_e(u, cb);
+        cell_e(e, ce);
+        o.bex = cb.ex;
+        o.bez = cb.ez;
+        o.buy = cb.uy;
+        o.bxez = right_of(cb.ez, ce.ez);
+        const int f[2] = {5, 10};
+        F2 w[2];
+        ld_fields<VEC>(F, n, f, r0 + kp, r1 + kp, w);
+        o.fx2 = w[0];      // x sweep bt2: Ey at the x face
+        o.fy1 = w[1];      // y sweep bt1: -Ex at the y face
+    };
+    Plane A;
+    load(k0 * plane, A);
+#pragma unroll 1
+    for (int k = k0; k < k1; ++k) {
+        const int kp = k * plane;
+        Plane B;
+        load(wrap_up(k, dm.nz) * plane, B);
+        const int fr[4] = {4, 11, 16, 17}, fq[2] = {4, 17}, fx[2] = {11, 16};
+        F2 w[4], wq[2];
+        F1 wx[2];
+        ld_fields<VEC>(F, n, fr, r0 + kp, r1 + kp, w);
+        ld_fields<VEC>(F, n, fq, q0 + kp, q1 + kp, wq);
+        ld_fields<VEC>(F, n, fx, r2 + kp, 0, wx);
+        const F2 neg = same<F2>(-1.0f), quarter = same<F2>(0.25f);
+        // Only the signs of the face velocities are used.  In a table, where one
+        // is near zero, the velocities are divided out as k_corner_emf divides,
+        // so that the same side is taken (0.14 ms more at 512^3).
+        F2 vx = A.a.ux + A.xux, vy = A.a.uy + A.buy, vz = A.a.uz + B.a.uz;
+        const float tol = ONE ? 0.0f : 1.0e-6f;
+        const bool near = near_zero(A.a.ux, A.xux, tol) || near_zero(A.a.uy, A.buy, tol) || near_zero(A.a.uz, B.a.uz, tol);
+        if (!ONE && near) {
+            const int kn = wrap_up(k, dm.nz) * plane;
+            auto vel = [&](int f, int c) { return fld(S, f, n)[c] / fld(S, 0, n)[c]; };
+            vx = pack2(vel(1, r0 + kp) + vel(1, r1 + kp), vel(1, r1 + kp) + vel(1, r2 + kp));
+            vy = pack2(vel(2, r0 + kp) + vel(2, q0 + kp), vel(2, r1 + kp) + vel(2, q1 + kp));
+            vz = pack2(vel(3, r0 + kp) + vel(3, r0 + kn), vel(3, r1 + kp) + vel(3, r1 + kn));
+        }
+        {   // Ez at (i+1/2, j+1/2, k)
+            const F2 X0 = neg * w[0], Xj = neg * wq[0], Y0 = w[1], Yx = right_of(w[1], wx[0]);
+            const F2 g = upwind_diff(vx, near, Y0 - A.a.ez, A.bez - Y0, Yx - A.xez, A.bxez - Yx);
+            const F2 h = upwind_diff(vy, near, X0 - A.a.ez, A.xez - X0, Xj - A.bez, A.bxez - Xj);
+            st_lanes<VEC>(E + 2 * (size_t)n, r0 + kp, r1 + kp, two, quarter * ((((X0 + Xj) + Y0) + Yx) + (g + h)));
+        }
+        {   // Ey at (i+1/2, j, k+1/2)
+            const F2 Z0 = neg * w[2], Zx = neg * right_of(w[2], wx[1]), X0 = A.fx2, X1 = B.fx2;
+            const F2 g = upwind_diff(vx, near, Z0 - A.a.ey, B.a.ey - Z0, Zx - A.xey, B.xey - Zx);
+            const F2 h = upwind_diff(vz, near, X0 - A.a.ey, A.xey - X0, X1 - B.a.ey, B.xey - X1);
+            st_lanes<VEC>(E + (size_t)n, r0 + kp, r1 + kp, two, quarter * ((((X0 + X1) + Z0) + Zx) + (g + h)));
+        }
+        {   // Ex at (i, j+1/2, k+1/2)
+            const F2 Z0 = w[3], Zj = wq[1], Y0 = neg * A.fy1, Y1 = neg * B.fy1;
+            const F2 g = upwind_diff(vy, near, Z0 - A.a.ex, B.a.ex - Z0, Zj - A.bex, B.bex - Zj);
+            const F2 h = upwind_diff(vz, near, Y0 - A.a.ex, A.bex - Y0, Y1 - B.a.ex, B.bex - Y1);
+            st_lanes<VEC>(E, r0 + kp, r1 + kp, two, quarter * ((((Y0 + Y1) + Z0) + Zj) + (g + h)));
+        }
+        A = B;
+    }
+}
+template <bool ONE, bool PROT>
+__global__ void __launch_bounds__(kBX, 4) k_corner_emf_f32(BatchArgs ba, int half_step_state) {
+    int local;
+    const BoxRec rp = resolve<ONE>(ba, kKindPairZ, local);
+    if (!rp.active || (PROT && !rp.protect)) return;
+    if (rp.vec) do_corner_emf_f32<ONE, PROT, true>(rp, local, half_step_state);
+    else do_corner_emf_f32<ONE, PROT, false>(rp, local, half_step_state);
+}
+
 // ============================================================ update
 // update_hydro_state_3d + final_check_unphysical (vanleer_mod.f90:2080-2207,
 // 3243-3262) and update_CT_3d with the cell-centre average (:2211-2259).
@@ -854,7 +1497,7 @@ __device__ __forceinline__ bool update_by_tma(const BoxRec& r) {
 // ZR: some box of the table restricts its maxima to a z range (slabs); the
 // other instantiation has no per-plane test on the hot path.
 template <class T, bool ONE, bool ZR, bool SHORT = false>
-__global__ void __launch_bounds__(kBX, sizeof(T) == 4 ? 6 : 1) k_update(BatchArgs ba, double dt_scale, int final_stage) {
+__global__ void __launch_bounds__(kBX, 1) k_update(BatchArgs ba, double dt_scale, int final_stage) {
     int local;
     const BoxRec rp = resolve<ONE>(ba, kKindCellZ, local);
     Scalars* sc = rp.sc;
@@ -963,6 +1606,152 @@ __global__ void __launch_bounds__(kBX, sizeof(T) == 4 ? 6 : 1) k_update(BatchArg
     if (do_cfl) block_atomic_max<kBX>(cmax_slots, cmax);
 }
 
+// ------------------------------------------------------------ FP32 update
+// k_update on a pair of cells per thread (8-byte loads; the left neighbour of
+// the second cell is the first).  Bound by HBM: 128 B per cell at 6.7 TB/s (81%
+// of DRAM peak in ncu), 2.55 ms a launch at 512^3 and 0.63 at 320^3 for any row
+// length.  A cell's values are all finite when the sum
+// of their products with 0 is 0.
+template <class V>
+__device__ __forceinline__ V vt_pair(V rho0, V m0, V ir1, V m1) {
+    return same<V>(0.5f) * fma(m0, vrcp(rho0), m1 * ir1);
+}
+// cell_max_speed of a pair, with its operations
+__device__ __forceinline__ F2 cell_speed_fast(F2 rho, const F2* m, F2 bxc, F2 byc, F2 bzc, float asqr) {
+    const F2 is = each([](float r) { return 1.0f / sqrtf(r); }, rho), a2 = same<F2>(asqr);
+    const F2 bx = bxc * is, by = byc * is, bz = bzc * is, half = same<F2>(0.5f);
+    auto fast = [&](F2 bt, F2 n) {
+        const F2 b = fma(n, n, bt), d = a2 - b;
+        return vsqrt(half * ((a2 + b) + vsqrt(fma(d, d, same<F2>(4.0f * asqr) * bt))));
+    };
+    const F2 cx = fast(fma(by, by, bz * bz), bx), cy = fast(fma(bx, bx, bz * bz), by), cz = fast(fma(bx, bx, by * by), bz);
+    auto quot = [](float a, float b) { return a / b; };
+    return vmax2(vmax2(vabs(each(quot, m[0], rho)) + cx, vabs(each(quot, m[1], rho)) + cy), vabs(each(quot, m[2], rho)) + cz);
+}
+template <bool ONE, bool ZR, bool VEC>
+__device__ __forceinline__ void do_update_f32(const BoxRec& rp, int local, double dt_scale, int final_stage) {
+    Scalars* sc = rp.sc;
+    const Dims dm = dims_of(rp);
+    const float* __restrict__ S0 = (const float*)rp.S[0];
+    float* __restrict__ Sout = (float*)rp.S[1];
+    const float* __restrict__ F = (const float*)rp.F;
+    const float* __restrict__ E = (const float*)rp.E;
+    const float asqr = (float)(rp.cs * rp.cs);
+    const int do_cfl = final_stage && !sc->drive;
+    const bool write_vt = final_stage && rp.npass > 0;
+    int p, j, k0, k1;
+    decode_cellz<ONE, true>(local, Dims{pairs_of(dm.nx), dm.ny, dm.nz, 0}, rp.ptws, rp.segzs, p, j, k0, k1);
+    double cmax = 0.0;
+    if (2 * p < dm.nx && j < dm.ny) {
+        const int n = dm.n, plane = dm.nx * dm.ny;
+        const F2 ndt = same<F2>((float)(-dt_scale * sc->dt / rp.dx)), half = same<F2>(0.5f);
+        const int x0 = 2 * p, x1 = wrap_up(x0, dm.nx), xm = wrap_dn(x0, dm.nx), row = dm.nx * j, rowm = dm.nx * wrap_dn(j, dm.ny);
+        const bool two = x0 + 1 < dm.nx;
+        const int r0 = row + x0, r1 = row + x1, rm = row + xm, q0 = rowm + x0, q1 = rowm + x1, qm = rowm + xm;
+        // flux component of xyz variable v in sweep D: rho -> 0; momentum X -> 1 + (X - D) mod 3
+        const int ff[12] = {0, 1, 2, 3, 6, 9, 7, 8, 12, 14, 15, 13}, fxf[4] = {0, 1, 2, 3}, fyf[4] = {6, 9, 7, 8};
+        const int ef[3] = {0, 1, 2}, eq[2] = {0, 2}, ex[2] = {1, 2};
+        // values of plane k-1 (periodic image for the first cells of the column)
+        F2 Fzm[4], Ex_zm, Ey_zm, Ex_ymzm, Ey_xmzm, bzm;
+        {
+            const int km = wrap_dn(k0, dm.nz) * plane;
+            const int fz[4] = {12, 14, 15, 13}, e2[2] = {0, 1}, f9[1] = {9}, f0[1] = {0}, f1[1] = {1};
+            F2 e[2], b[1], eym[1];
+            F1 exm[1];
+            ld_fields<VEC>(F, n, fz, r0 + km, r1 + km, Fzm);
+            ld_fields<VEC>(E, n, e2, r0 + km, r1 + km, e);
+            ld_fields<VEC>(E, n, f0, q0 + km, q1 + km, eym);
+            ld_fields<VEC>(E, n, f1, rm + km, 0, exm);
+            ld_fields<VEC>(S0, n, f9, r0 + km, r1 + km, b);
+            Ex_zm = e[0];
+            Ey_zm = e[1];
+            Ex_ymzm = eym[0];
+            Ey_xmzm = left_of(e[1], exm[0]);
+            bzm = fma(ndt, (Ey_zm - Ey_xmzm) - (Ex_zm - Ex_ymzm), b[0]);
+        }
+#pragma unroll 1
+        for (int k = k0; k < k1; ++k) {
+            const int kp = k * plane, c0 = r0 + kp, c1 = r1 + kp;
+            const int sf[7] = {0, 1, 2, 3, 7, 8, 9}, f7[1] = {7}, f8[1] = {8};
+            F2 u[7], f[12], fy[4], e[3], eym[2], bym_[1];
+            F1 fxm[4], exm[2], eqm[1], bxm_[1];
+            ld_fields<VEC>(S0, n, sf, c0, c1, u);
+            ld_fields<VEC>(F, n, ff, c0, c1, f);
+            ld_fields<VEC>(F, n, fyf, q0 + kp, q1 + kp, fy);
+            ld_fields<VEC>(E, n, ef, c0, c1, e);
+            ld_fields<VEC>(E, n, eq, q0 + kp, q1 + kp, eym);
+            ld_fields<VEC>(S0, n, f8, q0 + kp, q1 + kp, bym_);
+            ld_fields<VEC>(F, n, fxf, rm + kp, 0, fxm);
+            ld_fields<VEC>(E, n, ex, rm + kp, 0, exm);
+            const int e2[1] = {2};
+            ld_fields<VEC>(E, n, e2, qm + kp, 0, eqm);
+            ld_fields<VEC>(S0, n, f7, rm + kp, 0, bxm_);
+            F2 out[4];
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+                const F2 d = (f[v] - left_of(f[v], fxm[v])) + (f[4 + v] - fy[v]) + (f[8 + v] - Fzm[v]);
+                out[v] = fma(ndt, d, u[v]);
+                Fzm[v] = f[8 + v];
+            }
+            const bool inz = !ZR || (k >= rp.zlo && k < rp.zhi);
+            if (any_less(out[0], same<F2>((float)kMIN_DENS))) {
+#pragma unroll 1
+                for (int l = 0; l < 2; ++l) {
+                    if (lane(out[0], l) < (float)kMIN_DENS) {
+                        set_lane(out[0], l, (float)kMIN_DENS);
+                        if (l == 0 || two) {
+                            if (rp.protect) prot_mark_bad(rp, final_stage, l ? c1 : c0);   // updated again by k_prot_hydro
+                            else if (inz) atomicAdd(&sc->floor_hits, 1ull);
+                        }
+                    }
+                }
+            }
+            const F2 Ey_xm = left_of(e[1], exm[0]), Ez_xm = left_of(e[2], exm[1]), Ez_xmym = left_of(eym[1], eqm[0]);
+            const F2 Ex_ym = eym[0], Ez_ym = eym[1];
+            // ct_bx / ct_by / ct_bz of the face fields at c and at the minus faces
+            const F2 bx = fma(ndt, (e[2] - Ez_ym) - (e[1] - Ey_zm), u[4]);
+            const F2 by = fma(ndt, (e[0] - Ex_zm) - (e[2] - Ez_xm), u[5]);
+            const F2 bz = fma(ndt, (e[1] - Ey_xm) - (e[0] - Ex_ym), u[6]);
+            const F2 bxm = fma(ndt, (Ez_xm - Ez_xmym) - (Ey_xm - Ey_xmzm), left_of(u[4], bxm_[0]));
+            const F2 bym = fma(ndt, (Ex_ym - Ex_ymzm) - (Ez_ym - Ez_xmym), bym_[0]);
+            const F2 bxc = half * (bx + bxm), byc = half * (by + bym), bzc = half * (bz + bzm);
+            const F2 so[10] = {out[0], out[1], out[2], out[3], bxc, byc, bzc, bx, by, bz};
+#pragma unroll
+            for (int v = 0; v < 10; ++v) st_lanes<VEC>(Sout + (size_t)v * n, c0, c1, two, so[v]);
+            if (final_stage) {
+                if (write_vt) {
+                    const F2 ir = vrcp(out[0]);
+#pragma unroll
+                    for (int d = 0; d < 3; ++d)
+                        st_lanes<VEC>(vt_field<float>(rp, d), c0, c1, two, vt_pair(u[0], u[1 + d], ir, out[1 + d]));
+                }
+                if (do_cfl && inz)
+                    cmax = nmax(cmax, (double)nan_top(cell_speed_fast(out[0], out + 1, bxc, byc, bzc, asqr)));
+            }
+            const F2 zero = same<F2>(0.0f);
+            F2 fin = out[0] * zero;
+#pragma unroll
+            for (int v = 1; v < 4; ++v) fin = fma(out[v], zero, fin);
+            fin = fma(bx, zero, fma(by, zero, fma(bz, zero, fin)));
+            if (inz && !(nan_top(fin) == 0.0f)) atomicOr(&sc->status, 2u);
+            Ex_zm = e[0];
+            Ey_zm = e[1];
+            Ex_ymzm = Ex_ym;
+            Ey_xmzm = Ey_xm;
+            bzm = bz;
+        }
+    }
+    if (do_cfl) block_atomic_max<kBX>(sc->cmax_slots, cmax);
+}
+template <bool ONE, bool ZR>
+__global__ void __launch_bounds__(kBX, 4) k_update_f32(BatchArgs ba, double dt_scale, int final_stage) {
+    int local;
+    const BoxRec rp = resolve<ONE>(ba, kKindPairZ, local);
+    if (!rp.active) return;
+    if (rp.vec) do_update_f32<ONE, ZR, true>(rp, local, dt_scale, final_stage);
+    else do_update_f32<ONE, ZR, false>(rp, local, dt_scale, final_stage);
+}
+
 // ------------------------------------------------------------ update, TMA-fed
 // The same update for boxes whose rows are whole 128-cell tiles (TW = 128),
 // or 64-cell tiles with an even row count (TW = 64, two rows per block): a
@@ -1027,7 +1816,7 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned by
 }
 
 template <class T, bool ZR, bool ONE, int TW>
-__global__ void __launch_bounds__(kTmaTile, sizeof(T) == 4 ? 6 : 1)
+__global__ void __launch_bounds__(kTmaTile, 1)
     k_update_tma(BatchArgs ba, double dt_scale, int final_stage) {
     extern __shared__ __align__(128) unsigned char tma_smem[];
     __shared__ __align__(8) unsigned long long bars[2];
@@ -1409,24 +2198,12 @@ __global__ void __launch_bounds__(kBX) k_prot_clear(BatchArgs ba, int stage) {
 }
 
 // ============================================================ passive scalars
-// Upwind flux of compute_fluxes_1d (passive_mod.f90:594-627).  The
-// reference's arithmetic form in FP32 too: a select of the upwind state
-// (equal for finite operands) lets the compiler fold the two neighbour loads
-// into one whose address waits on the velocity, and the z-marching passive
-// predictor went from 1.35 to 1.61 ms at 512^3.
+// Upwind flux of compute_fluxes_1d (passive_mod.f90:594-627), the reference's
+// arithmetic form.
 template <class T>
 __device__ __forceinline__ T upwind_flux(T uL, T uR, T vavg) {
     T theta = (vavg >= T(0)) ? T(1) : T(-1);
     return T(0.5) * ((T(1) + theta) * uL + (T(1) - theta) * uR);
-}
-// The same flux where both states come from shared memory (the bulk-copy
-// fed passive kernels): FP32 selects the upwind state, equal to the form
-// above for finite operands, and there the select is cheaper (bulk-copy fed
-// corrector 2.20 -> 2.05 ms at 512^3).
-template <class T>
-__device__ __forceinline__ T upwind_sel(T uL, T uR, T vavg) {
-    if constexpr (sizeof(T) == 4) return (vavg >= T(0)) ? uL : uR;
-    else return upwind_flux(uL, uR, vavg);
 }
 template <class T>
 __device__ __forceinline__ T vel_of(const T* __restrict__ S, int n, int c, int comp) {
@@ -1439,11 +2216,9 @@ __device__ __forceinline__ T vel_of(const T* __restrict__ S, int n, int c, int c
 // 133-157, 204-224, 562-590).
 // A thread walks a column of kSegZ cells along z, carrying the z velocity
 // and the flux through the lower z face (the upper face's of the previous
-// cell: the same operands).  The neighbour loads are
-// latency-bound, so FP32 with up to four scalars runs eight blocks per SM
-// (64 registers).
+// cell: the same operands).  FP64; FP32 runs k_passive_pred_f32.
 template <class T, bool ONE, int NP, bool SHORT = false>
-__global__ void __launch_bounds__(kBX, (sizeof(T) == 4 && NP <= 4) ? 8 : 1) k_passive_pred(BatchArgs ba) {
+__global__ void __launch_bounds__(kBX, 1) k_passive_pred(BatchArgs ba) {
     int local;
     const BoxRec rp = resolve<ONE>(ba, kKindCellZ, local);
     const Scalars* sc = rp.sc;
@@ -1529,10 +2304,9 @@ __device__ __forceinline__ T vtavg(const T* __restrict__ S0, const T* __restrict
 // A thread walks a column of kSegZ cells along z, carrying the z-neighbour
 // time-averaged velocity, half-step scalars, their minmod slopes and the
 // flux through the lower z face (the upper face's of the previous cell).
-// Eight blocks per SM in FP32 with up to four scalars, as k_passive_pred
-// (a few spilled values cost less than the lost occupancy).
+// FP64; FP32 runs k_passive_corr_f32.
 template <class T, bool ONE, int NP, bool SHORT = false>
-__global__ void __launch_bounds__(kBX, (sizeof(T) == 4 && NP <= 4) ? 8 : 1) k_passive_corr(BatchArgs ba) {
+__global__ void __launch_bounds__(kBX, 1) k_passive_corr(BatchArgs ba) {
     int local;
     const BoxRec rp = resolve<ONE>(ba, kKindCellZ, local);
     const Scalars* sc = rp.sc;
@@ -1635,6 +2409,253 @@ __global__ void __launch_bounds__(kBX, (sizeof(T) == 4 && NP <= 4) ? 8 : 1) k_pa
         }
         vz_0 = vz_p;
     }
+}
+
+// ------------------------------------------------------ FP32 passive scalars
+// k_passive_pred and k_passive_corr on a pair of cells per thread: the pair
+// shares the velocities, slopes and fluxes of its inner x face, rows are read
+// 8 bytes at a time, and the upwind state is selected (equal to upwind_flux
+// for finite operands).  Bound by latency (13 long-scoreboard stalls per issue
+// before the loads of two scalars were put together): predictor 0.78 ms, 5.5
+// TB/s of the algorithmic 32 B per cell, corrector 1.95 ms at 512^3 with two
+// scalars.
+__device__ __forceinline__ F2 upwind_pick(F2 uL, F2 uR, F2 v) { return vsel(v, uL, uR); }
+// minmod, from the signed minima (the same values)
+template <class V>
+__device__ __forceinline__ V minmod_fast(V wm, V w0, V wp) {
+    return each([](float m, float c, float p) {
+        const float a = __fsub_rn(c, m), b = __fsub_rn(p, c);
+        return __fadd_rn(fmaxf(fminf(a, b), 0.0f), fminf(fmaxf(a, b), 0.0f));
+    }, wm, w0, wp);
+}
+template <bool ONE, int NP, bool VEC>
+__device__ __forceinline__ void do_passive_pred_f32(const BoxRec& rp, int local) {
+    const Scalars* sc = rp.sc;
+    const int npass = rp.npass;
+    const Dims dm = dims_of(rp);
+    const float* __restrict__ S0 = (const float*)rp.S[0];
+    float* __restrict__ SH = (float*)rp.SH;
+    int p, j, k0, k1;
+    decode_cellz<ONE, true>(local, Dims{pairs_of(dm.nx), dm.ny, dm.nz, 0}, rp.ptws, rp.segzs, p, j, k0, k1);
+    if (2 * p >= dm.nx || j >= dm.ny) return;
+    const int n = dm.n, plane = dm.nx * dm.ny;
+    const F2 ndt = same<F2>((float)(-0.5 * sc->dt / rp.dx)), half = same<F2>(0.5f);
+    const int x0 = 2 * p, x1 = wrap_up(x0, dm.nx), x2 = wrap_up(x1, dm.nx), xm = wrap_dn(x0, dm.nx);
+    const bool two = x0 + 1 < dm.nx;
+    const int row = dm.nx * j, rowm = dm.nx * wrap_dn(j, dm.ny), rowp = dm.nx * wrap_up(j, dm.ny);
+    const int vz2[2] = {0, 3}, vy2[2] = {0, 2}, vx2[2] = {0, 1}, all[4] = {0, 1, 2, 3};
+    F2 vz_0, s_0[NP], fz_m[NP];
+    {
+        const int ckm = wrap_dn(k0, dm.nz) * plane, ck0 = k0 * plane;
+        F2 a[2], b[2];
+        ld_fields<VEC>(S0, n, vz2, row + x0 + ckm, row + x1 + ckm, a);
+        ld_fields<VEC>(S0, n, vz2, row + x0 + ck0, row + x1 + ck0, b);
+        const F2 vz_m = a[1] * vrcp(a[0]);
+        vz_0 = b[1] * vrcp(b[0]);
+#pragma unroll
+        for (int q = 0; q < NP; ++q)
+            {
+                const float* s = S0 + (size_t)(10 + min(q, npass - 1)) * n;
+                s_0[q] = ld_lanes<F2, VEC>(s, row + x0 + ck0, row + x1 + ck0);
+                fz_m[q] = upwind_pick(ld_lanes<F2, VEC>(s, row + x0 + ckm, row + x1 + ckm), s_0[q], half * (vz_m + vz_0));
+            }
+    }
+#pragma unroll 1
+    for (int k = k0; k < k1; ++k) {
+        const int kp = k * plane, kz = wrap_up(k, dm.nz) * plane;
+        F2 u[4], a[2], b[2], z[2];
+        F1 l[2], r[2];
+        ld_fields<VEC>(S0, n, all, row + x0 + kp, row + x1 + kp, u);
+        ld_fields<VEC>(S0, n, vy2, rowm + x0 + kp, rowm + x1 + kp, a);
+        ld_fields<VEC>(S0, n, vy2, rowp + x0 + kp, rowp + x1 + kp, b);
+        ld_fields<VEC>(S0, n, vz2, row + x0 + kz, row + x1 + kz, z);
+        ld_fields<VEC>(S0, n, vx2, row + xm + kp, 0, l);
+        ld_fields<VEC>(S0, n, vx2, row + x2 + kp, 0, r);
+        const F2 ir = vrcp(u[0]), vx0 = u[1] * ir, vy0 = u[2] * ir;
+        const F2 fxm = half * (left_of(vx0, l[1] * vrcp(l[0])) + vx0), fxp = half * (vx0 + right_of(vx0, r[1] * vrcp(r[0])));
+        const F2 fym = half * (a[1] * vrcp(a[0]) + vy0), fyp = half * (vy0 + b[1] * vrcp(b[0]));
+        const F2 vz_p = z[1] * vrcp(z[0]), fzp = half * (vz_0 + vz_p);
+        // two scalars at a time, their loads first (a scalar past npass repeats
+        // the last one and stores nothing)
+#pragma unroll
+        for (int g = 0; g < NP; g += 2) {
+            constexpr int G = NP < 2 ? 1 : 2;
+            F1 sl[G], sr[G];
+            F2 sym[G], syp[G], s_zp[G];
+#pragma unroll
+            for (int h = 0; h < G; ++h) {
+                if (g + h >= NP) break;
+                const float* s = S0 + (size_t)(10 + min(g + h, npass - 1)) * n;
+                sl[h] = ld_lanes<F1, VEC>(s, row + xm + kp, 0);
+                sr[h] = ld_lanes<F1, VEC>(s, row + x2 + kp, 0);
+                sym[h] = ld_lanes<F2, VEC>(s, rowm + x0 + kp, rowm + x1 + kp);
+                syp[h] = ld_lanes<F2, VEC>(s, rowp + x0 + kp, rowp + x1 + kp);
+                s_zp[h] = ld_lanes<F2, VEC>(s, row + x0 + kz, row + x1 + kz);
+            }
+#pragma unroll
+            for (int h = 0; h < G; ++h) {
+                const int q = g + h;
+                if (q >= NP) break;
+                const F2 s0 = s_0[q];
+                const F2 dx = upwind_pick(s0, right_of(s0, sr[h]), fxp) - upwind_pick(left_of(s0, sl[h]), s0, fxm);
+                const F2 dy = upwind_pick(s0, syp[h], fyp) - upwind_pick(sym[h], s0, fym);
+                const F2 fz = upwind_pick(s0, s_zp[h], fzp), dz = fz - fz_m[q];
+                if (q < npass)
+                    st_lanes<VEC>(SH + (size_t)q * n, row + x0 + kp, row + x1 + kp, two,
+                                  fma(ndt, fma(vz_0, dz, fma(vx0, dx, vy0 * dy)), s0));
+                s_0[q] = s_zp[h];
+                fz_m[q] = fz;
+            }
+        }
+        vz_0 = vz_p;
+    }
+}
+template <bool ONE, int NP>
+__global__ void __launch_bounds__(kBX, NP <= 2 ? 8 : NP <= 4 ? 6 : 3) k_passive_pred_f32(BatchArgs ba) {
+    int local;
+    const BoxRec rp = resolve<ONE>(ba, kKindPairZ, local);
+    if (!rp.active || rp.npass == 0) return;
+    if (rp.vec) do_passive_pred_f32<ONE, NP, true>(rp, local);
+    else do_passive_pred_f32<ONE, NP, false>(rp, local);
+}
+
+template <bool ONE, int NP, bool VEC>
+__device__ __forceinline__ void do_passive_corr_f32(const BoxRec& rp, int local) {
+    const Scalars* sc = rp.sc;
+    const int npass = rp.npass;
+    const Dims dm = dims_of(rp);
+    const float* __restrict__ S0 = (const float*)rp.S[0];
+    float* __restrict__ S1 = (float*)rp.S[1];
+    const float* __restrict__ SH = (const float*)rp.SH;
+    const float* __restrict__ VT = vt_field<float>(rp, 0);   // fields 0, 1 at +0, +n; field 2 at +6n (vt_field)
+    const int drive = sc->drive, plane_stride = rp.plane_stride;
+    const float* __restrict__ mbnd = (const float*)rp.mbnd;
+    int p, j, k0, k1;
+    decode_cellz<ONE, true>(local, Dims{pairs_of(dm.nx), dm.ny, dm.nz, 0}, rp.ptws, rp.segzs, p, j, k0, k1);
+    if (2 * p >= dm.nx || j >= dm.ny) return;
+    const int n = dm.n, plane = dm.nx * dm.ny;
+    const F2 ndt = same<F2>((float)(-sc->dt / rp.dx)), half = same<F2>(0.5f);
+    const int x0 = 2 * p, x1 = wrap_up(x0, dm.nx), x2 = wrap_up(x1, dm.nx), x3 = wrap_up(x2, dm.nx);
+    const int xm = wrap_dn(x0, dm.nx), xm2 = wrap_dn(xm, dm.nx);
+    const bool two = x0 + 1 < dm.nx;
+    const int jm = wrap_dn(j, dm.ny), jp = wrap_up(j, dm.ny);
+    const int row = dm.nx * j, rowm = dm.nx * jm, rowp = dm.nx * jp;
+    const int rowm2 = dm.nx * wrap_dn(jm, dm.ny), rowp2 = dm.nx * wrap_up(jp, dm.ny);
+    // on drive steps the velocity across the global boundary of axis d uses
+    // the unforced momentum of the ghost image (mbnd planes, see k_force_kick)
+    auto ghost = [&](int c, int comp, int side, int ofs) {
+        return vtavg(S0, S1, VT, n, c, comp, mbnd + (size_t)(2 * comp + side) * plane_stride + ofs);
+    };
+    auto zghost = [&](int kk, int side) {
+        return pack2(ghost(row + x0 + kk * plane, 2, side, row + x0), ghost(row + x1 + kk * plane, 2, side, row + x1));
+    };
+    const float* VZ = VT + (size_t)6 * n;
+    const int km = wrap_dn(k0, dm.nz);
+    F2 vz_0 = ld_lanes<F2, VEC>(VZ, row + x0 + k0 * plane, row + x1 + k0 * plane);
+    F2 s_0[NP], s_p[NP], hi_0[NP], fz_m[NP];    // hi: s + slope / 2 of cell k
+    {
+        const F2 vz_m = drive && k0 == 0 ? zghost(km, 1) : ld_lanes<F2, VEC>(VZ, row + x0 + km * plane, row + x1 + km * plane);
+        const int km2 = wrap_dn(km, dm.nz) * plane, kp = wrap_up(k0, dm.nz) * plane;
+#pragma unroll
+        for (int q = 0; q < NP; ++q)
+            {
+                const float* s = SH + (size_t)min(q, npass - 1) * n;
+                const F2 sm2 = ld_lanes<F2, VEC>(s, row + x0 + km2, row + x1 + km2);
+                const F2 sm = ld_lanes<F2, VEC>(s, row + x0 + km * plane, row + x1 + km * plane);
+                s_0[q] = ld_lanes<F2, VEC>(s, row + x0 + k0 * plane, row + x1 + k0 * plane);
+                s_p[q] = ld_lanes<F2, VEC>(s, row + x0 + kp, row + x1 + kp);
+                const F2 dm_ = half * minmod_fast(sm2, sm, s_0[q]), d0 = half * minmod_fast(sm, s_0[q], s_p[q]);
+                hi_0[q] = s_0[q] + d0;
+                fz_m[q] = upwind_pick(sm + dm_, s_0[q] - d0, half * (vz_m + vz_0));
+            }
+    }
+#pragma unroll 1
+    for (int k = k0; k < k1; ++k) {
+        const int kp = k * plane, kz = wrap_up(k, dm.nz) * plane, kz2 = wrap_up(wrap_up(k, dm.nz), dm.nz) * plane;
+        const int c0 = row + x0 + kp, c1 = row + x1 + kp;
+        const F2 vx0 = ld_lanes<F2, VEC>(VT, c0, c1), vy0 = ld_lanes<F2, VEC>(VT + n, c0, c1);
+        F1 vl = ld_lanes<F1, VEC>(VT, row + xm + kp, 0), vr = ld_lanes<F1, VEC>(VT, row + x2 + kp, 0);
+        F2 vym = ld_lanes<F2, VEC>(VT + n, rowm + x0 + kp, rowm + x1 + kp);
+        F2 vyp = ld_lanes<F2, VEC>(VT + n, rowp + x0 + kp, rowp + x1 + kp);
+        F2 vz_p = ld_lanes<F2, VEC>(VZ, row + x0 + kz, row + x1 + kz);
+        F2 vxp = right_of(vx0, vr);
+        if (drive) {
+            const int px = j + dm.ny * k, py = dm.nx * k;
+            if (x0 == 0) vl.v = ghost(row + xm + kp, 0, 1, px);
+            if (x0 == dm.nx - 1) set_lane(vxp, 0, ghost(row + x1 + kp, 0, 0, px));
+            if (x0 + 1 == dm.nx - 1) set_lane(vxp, 1, ghost(row + x2 + kp, 0, 0, px));
+            if (j == 0) vym = pack2(ghost(rowm + x0 + kp, 1, 1, x0 + py), ghost(rowm + x1 + kp, 1, 1, x1 + py));
+            if (j == dm.ny - 1) vyp = pack2(ghost(rowp + x0 + kp, 1, 0, x0 + py), ghost(rowp + x1 + kp, 1, 0, x1 + py));
+            if (k == dm.nz - 1) vz_p = zghost(0, 0);
+        }
+        const F2 fxm = half * (left_of(vx0, vl) + vx0), fxp = half * (vx0 + vxp);
+        const F2 fym = half * (vym + vy0), fyp = half * (vy0 + vyp), fzp = half * (vz_0 + vz_p);
+        // loads of two scalars first, as in the predictor
+#pragma unroll
+        for (int g = 0; g < NP; g += 2) {
+            constexpr int G = NP < 2 ? 1 : 2;
+            F1 xa[G], xb[G], xc[G], xd[G];
+            F2 sm[G], sp[G], sm2[G], sp2[G], szz[G], base[G];
+#pragma unroll
+            for (int h = 0; h < G; ++h) {
+                if (g + h >= NP) break;
+                const int q = min(g + h, npass - 1);
+                const float* s = SH + (size_t)q * n;
+                xa[h] = ld_lanes<F1, VEC>(s, row + xm2 + kp, 0);
+                xb[h] = ld_lanes<F1, VEC>(s, row + xm + kp, 0);
+                xc[h] = ld_lanes<F1, VEC>(s, row + x2 + kp, 0);
+                xd[h] = ld_lanes<F1, VEC>(s, row + x3 + kp, 0);
+                sm[h] = ld_lanes<F2, VEC>(s, rowm + x0 + kp, rowm + x1 + kp);
+                sp[h] = ld_lanes<F2, VEC>(s, rowp + x0 + kp, rowp + x1 + kp);
+                sm2[h] = ld_lanes<F2, VEC>(s, rowm2 + x0 + kp, rowm2 + x1 + kp);
+                sp2[h] = ld_lanes<F2, VEC>(s, rowp2 + x0 + kp, rowp2 + x1 + kp);
+                szz[h] = ld_lanes<F2, VEC>(s, row + x0 + kz2, row + x1 + kz2);
+                base[h] = ld_lanes<F2, VEC>(S0 + (size_t)(10 + q) * n, c0, c1);
+            }
+#pragma unroll
+            for (int h = 0; h < G; ++h) {
+                const int q = g + h;
+                if (q >= NP) break;
+                const F2 s0 = s_0[q];
+                F2 dF[3];
+                {
+                    float p0, p1;
+                    unpack2(s0, p0, p1);
+                    const F2 d = half * minmod_fast(left_of(s0, xb[h]), s0, right_of(s0, xc[h]));
+                    const F1 h1 = same<F1>(0.5f);
+                    const F1 gl = h1 * minmod_fast(xa[h], xb[h], F1{p0}), gr = h1 * minmod_fast(F1{p1}, xc[h], xd[h]);
+                    const F2 hi = s0 + d, lo = s0 - d;
+                    dF[0] = upwind_pick(hi, right_of(lo, xc[h] - gr), fxp) - upwind_pick(left_of(hi, xb[h] + gl), lo, fxm);
+                }
+                {
+                    const F2 d = half * minmod_fast(sm[h], s0, sp[h]), gm = half * minmod_fast(sm2[h], sm[h], s0);
+                    const F2 gp = half * minmod_fast(s0, sp[h], sp2[h]);
+                    dF[1] = upwind_pick(s0 + d, sp[h] - gp, fyp) - upwind_pick(sm[h] + gm, s0 - d, fym);
+                }
+                {
+                    const F2 up = s_p[q], gp = half * minmod_fast(s0, up, szz[h]);
+                    const F2 Fp = upwind_pick(hi_0[q], up - gp, fzp);
+                    dF[2] = Fp - fz_m[q];
+                    fz_m[q] = Fp;
+                    s_0[q] = up;
+                    s_p[q] = szz[h];
+                    hi_0[q] = up + gp;
+                }
+                if (q < npass)
+                    st_lanes<VEC>(S1 + (size_t)(10 + q) * n, c0, c1, two,
+                                  fma(ndt, fma(vz_0, dF[2], fma(vx0, dF[0], vy0 * dF[1])), base[h]));
+            }
+        }
+        vz_0 = vz_p;
+    }
+}
+template <bool ONE, int NP>
+__global__ void __launch_bounds__(kBX, NP <= 2 ? 5 : NP <= 4 ? 3 : 2) k_passive_corr_f32(BatchArgs ba) {
+    int local;
+    const BoxRec rp = resolve<ONE>(ba, kKindPairZ, local);
+    if (!rp.active || rp.npass == 0) return;
+    if (rp.vec) do_passive_corr_f32<ONE, NP, true>(rp, local);
+    else do_passive_corr_f32<ONE, NP, false>(rp, local);
 }
 
 // ------------------------------------------------------ passive corrector, bulk-copy fed
@@ -1805,21 +2826,21 @@ __global__ void __launch_bounds__(kTmaTile, 8) k_passive_corr_tma(BatchArgs ba) 
                 {
                     const T sm = at(rj, -1), sp = at(rj, 1), sm2 = at(rj, -2), sp2 = at(rj, 2);
                     const T dlm = minmod(sm2, sm, s0), dl0 = minmod(sm, s0, sp), dlp = minmod(s0, sp, sp2);
-                    const T Fp = upwind_sel(s0 + T(0.5) * dl0, sp - T(0.5) * dlp, T(0.5) * (vx0 + vxp));
-                    const T Fm = upwind_sel(sm + T(0.5) * dlm, s0 - T(0.5) * dl0, T(0.5) * (vxm + vx0));
+                    const T Fp = upwind_flux(s0 + T(0.5) * dl0, sp - T(0.5) * dlp, T(0.5) * (vx0 + vxp));
+                    const T Fm = upwind_flux(sm + T(0.5) * dlm, s0 - T(0.5) * dl0, T(0.5) * (vxm + vx0));
                     dF[0] = Fp - Fm;
                 }
                 {
                     const T sm = at(rj - 1, 0), sp = at(rj + 1, 0), sm2 = at(rj - 2, 0), sp2 = at(rj + 2, 0);
                     const T dlm = minmod(sm2, sm, s0), dl0 = minmod(sm, s0, sp), dlp = minmod(s0, sp, sp2);
-                    const T Fp = upwind_sel(s0 + T(0.5) * dl0, sp - T(0.5) * dlp, T(0.5) * (vy0 + vyp));
-                    const T Fm = upwind_sel(sm + T(0.5) * dlm, s0 - T(0.5) * dl0, T(0.5) * (vym + vy0));
+                    const T Fp = upwind_flux(s0 + T(0.5) * dl0, sp - T(0.5) * dlp, T(0.5) * (vy0 + vyp));
+                    const T Fm = upwind_flux(sm + T(0.5) * dlm, s0 - T(0.5) * dl0, T(0.5) * (vym + vy0));
                     dF[1] = Fp - Fm;
                 }
                 {
                     const T sp = s_p[p], sp2 = at(6 * npass + 4 + p, 0);
                     const T dl0 = dl_0[p], dlp = minmod(s0, sp, sp2);
-                    const T Fp = upwind_sel(s0 + T(0.5) * dl0, sp - T(0.5) * dlp, T(0.5) * (vz_0 + vz_p));
+                    const T Fp = upwind_flux(s0 + T(0.5) * dl0, sp - T(0.5) * dlp, T(0.5) * (vz_0 + vz_p));
                     dF[2] = Fp - fz_m[p];
                     fz_m[p] = Fp;
                     s_0[p] = sp;
@@ -1860,10 +2881,9 @@ constexpr size_t ppred_stage_bytes() {
 template <class T, int NP>
 constexpr size_t passive_pred_tma_smem_bytes() { return 2 * ppred_stage_bytes<T, NP>(); }
 
-// FP32 occupancy: ten blocks per SM with up to two scalars (47 registers, no
-// spills: 1.32 -> 1.21 ms at 512^3), eight with four (ten spill).
+// FP64.
 template <class T, int NP>
-__global__ void __launch_bounds__(kTmaTile, sizeof(T) == 4 ? (NP <= 2 ? 10 : NP <= 4 ? 8 : 1) : 1)
+__global__ void __launch_bounds__(kTmaTile, 1)
     k_passive_pred_tma(BatchArgs ba) {
     extern __shared__ __align__(128) unsigned char pptma_smem[];
     __shared__ __align__(8) unsigned long long bars[2];
@@ -1964,9 +2984,9 @@ __global__ void __launch_bounds__(kTmaTile, sizeof(T) == 4 ? (NP <= 2 ? 10 : NP 
                 const int rs = 8 + p;
                 const T s0 = at(rs, 0), sxm = at(rs, -1), sxp = at(rs, 1);
                 const T sym = at(rs + NP, 0), syp = at(rs + 2 * NP, 0);
-                const T dfx = upwind_sel(s0, sxp, T(0.5) * (vx0 + vxp)) - upwind_sel(sxm, s0, T(0.5) * (vxm + vx0));
-                const T dfy = upwind_sel(s0, syp, T(0.5) * (vy0 + vyp)) - upwind_sel(sym, s0, T(0.5) * (vym + vy0));
-                const T fz = upwind_sel(ps[p], s0, T(0.5) * (pvz + vz0));   // face k-1/2
+                const T dfx = upwind_flux(s0, sxp, T(0.5) * (vx0 + vxp)) - upwind_flux(sxm, s0, T(0.5) * (vxm + vx0));
+                const T dfy = upwind_flux(s0, syp, T(0.5) * (vy0 + vyp)) - upwind_flux(sym, s0, T(0.5) * (vym + vy0));
+                const T fz = upwind_flux(ps[p], s0, T(0.5) * (pvz + vz0));   // face k-1/2
                 if (k > k0) fld(SH, p, n)[c - plane] = ps[p] - dtdx * (pvx * pdx[p] + pvy * pdy[p] + pvz * (fz - pfz[p]));
                 ps[p] = s0;
                 pdx[p] = dfx;

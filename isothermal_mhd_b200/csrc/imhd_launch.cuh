@@ -40,25 +40,26 @@ inline void mark(BatchDev& b, int stage) {
 
 // Grid of a launch of decomposition `kind`: the table's total block count, or
 // for a single box the 3D grid whose block indices the kernels read directly.
+// pairs: the kernel's threads take two cells along x (FP32 sweeps), its blocks
+// two rows in the x-row sweep.
 template <bool ONE>
-static dim3 grid_of(const BatchDev& b, int kind) {
+static dim3 grid_of(const BatchDev& b, int kind, bool pairs = false) {
     if constexpr (!ONE) {
         return dim3((unsigned)b.totals[kind]);
     } else {
         const BoxRec& r = b.a.one;
-        const int tw = 1 << r.tws, th = kBX >> r.tws;
-        unsigned nbx = (unsigned)((r.nx + tw - 1) / tw), nby = (unsigned)((r.ny + th - 1) / th);
+        const int tws = pairs ? r.ptws : r.tws, tw = 1 << tws, th = kBX >> tws, nu = pairs ? pairs_of(r.nx) : r.nx;
+        unsigned nbx = (unsigned)((nu + tw - 1) / tw), nby = (unsigned)((r.ny + th - 1) / th);
         unsigned nbz = (unsigned)((r.nz + th - 1) / th);
         if (kind == kKindCell) return dim3(nbx, nby, r.nz);
-        const int sz = 1 << r.segzs, sg = 1 << r.segs;
-        if (kind == kKindCellZ) return dim3(nbx, nby, (unsigned)((r.nz + sz - 1) / sz));
+        if (kind == kKindCellZ || kind == kKindPairZ) return dim3(nbx, nby, (unsigned)ceil_shift(r.nz, r.segzs));
         if (kind == kKindRed) return dim3((unsigned)r.nred);
         switch ((kind - kKindSolver0) % 5) {
-            case kSubCell: return dim3(nbx, nby, (unsigned)((r.nz + sz - 1) / sz));   // z columns
-            case kSubXRow: return dim3(r.ny, r.nz);
+            case kSubCell: return dim3(nbx, nby, (unsigned)ceil_shift(r.nz, r.segzs));   // z columns
+            case kSubXRow: return dim3((unsigned)(pairs ? (r.ny + 1) / 2 : r.ny), r.nz);
             case kSubXTile: return dim3((unsigned)((r.nx + kTX - 1) / kTX), r.ny, r.nz);
-            case kSubMarchY: return dim3(nbx, nbz, (unsigned)((r.ny + sg - 1) / sg));
-            default: return dim3(nbx, nby, (unsigned)((r.nz + sg - 1) / sg));
+            case kSubMarchY: return dim3(nbx, nbz, (unsigned)ceil_shift(r.ny, r.segs));
+            default: return dim3(nbx, nby, (unsigned)ceil_shift(r.nz, r.segs));
         }
     }
 }
@@ -70,35 +71,60 @@ static bool short_columns(const BatchDev& b) {
     return ONE && b.a.one.segzs < kSegZLog;
 }
 
+// Grid of the z-column cell kernels: tiles of cell pairs in FP32.
+template <class T, bool ONE>
+static dim3 zgrid(const BatchDev& b) {
+    return sizeof(T) == 4 ? grid_of<ONE>(b, kKindPairZ, true) : grid_of<ONE>(b, kKindCellZ);
+}
+
 // Corner EMFs of one stage (PROT: of the protection fluxes).
 template <class T, bool ONE, bool PROT>
 static void launch_emf(BatchDev& b, dim3 gz, int half_step_state) {
-    if constexpr (ONE) {
-        if (short_columns<ONE>(b)) {
-            k_corner_emf<T, ONE, PROT, true><<<gz, kBX, 0, b.st>>>(b.a, half_step_state);
-            b.launches += 1;
-            return;
-        }
-    }
-    k_corner_emf<T, ONE, PROT><<<gz, kBX, 0, b.st>>>(b.a, half_step_state);
     b.launches += 1;
+    if constexpr (sizeof(T) == 4) {
+        k_corner_emf_f32<ONE, PROT><<<gz, kBX, 0, b.st>>>(b.a, half_step_state);
+    } else {
+        if constexpr (ONE) {
+            if (short_columns<ONE>(b)) {
+                k_corner_emf<T, ONE, PROT, true><<<gz, kBX, 0, b.st>>>(b.a, half_step_state);
+                return;
+            }
+        }
+        k_corner_emf<T, ONE, PROT><<<gz, kBX, 0, b.st>>>(b.a, half_step_state);
+    }
 }
+
+// The flux kernels of a scheme that take two interfaces per thread (pair_fluxes,
+// pair_sweeps): FP32, but for the Roe boxes of a table; sweeps with PLM.
+template <class T, int SCHEME, bool ONE>
+constexpr bool pair_scheme() { return sizeof(T) == 4 && (ONE || scheme_solver(SCHEME) % 3 != 1); }
+template <class T, int SCHEME, bool ONE>
+constexpr bool pair_sweep() { return pair_scheme<T, SCHEME, ONE>() && !(scheme_recon(SCHEME) & 1); }
 
 template <class T, int SCHEME, bool ONE>
 static void launch_fluxes_pred(BatchDev& b) {
-    if (!b.has_scheme[SCHEME] || b.totals[scheme_kind(SCHEME, kSubCell)] == 0) return;
-    dim3 g = grid_of<ONE>(b, scheme_kind(SCHEME, kSubCell));
-    if constexpr (ONE) {
-        if (short_columns<ONE>(b)) {
-            k_pred_flux<T, SCHEME, ONE, true><<<g, kBX, 0, b.st>>>(b.a);
-            b.launches += 1;
-            return;
-        }
-    }
-    k_pred_flux<T, SCHEME, ONE><<<g, kBX, 0, b.st>>>(b.a);
+    const int kind = scheme_kind(SCHEME, kSubCell);
+    if (!b.has_scheme[SCHEME] || b.totals[kind] == 0) return;
     b.launches += 1;
+    if constexpr (pair_scheme<T, SCHEME, ONE>()) {
+        k_pred_flux_f32<scheme_solver(SCHEME), ONE><<<grid_of<ONE>(b, kind, true), kBX, 0, b.st>>>(b.a, kind);
+    } else {
+        if constexpr (ONE) {
+            if (short_columns<ONE>(b)) {
+                k_pred_flux<T, SCHEME, ONE, true><<<grid_of<ONE>(b, kind), kBX, 0, b.st>>>(b.a);
+                return;
+            }
+        }
+        k_pred_flux<T, SCHEME, ONE><<<grid_of<ONE>(b, kind), kBX, 0, b.st>>>(b.a);
+    }
 }
 
+// The x-row sweep of a scheme, two rows per block (PAIR) or one.
+template <class T, int SCHEME, bool ONE, bool PAIR>
+static auto xrow_kernel() {
+    if constexpr (pair_scheme<T, SCHEME, ONE>()) return &k_xrow_f32<SCHEME, std::conditional_t<PAIR, F2, F1>, ONE>;
+    else return &k_corr_flux_xrow<T, SCHEME, ONE>;
+}
 // The x-row sweep needs more than 48 KiB of dynamic shared memory for long
 // rows; the opt-in is per kernel and device and is done outside any capture.
 template <class T, int SCHEME, bool ONE>
@@ -107,7 +133,9 @@ static void ensure_xrow_attr() {
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64 || !attr_set[dev]) {
-        cudaFuncSetAttribute(k_corr_flux_xrow<T, SCHEME, ONE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowSmemMax);
+        cudaFuncSetAttribute(xrow_kernel<T, SCHEME, ONE, false>(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowSmemMax);
+        if constexpr (pair_sweep<T, SCHEME, ONE>())
+            cudaFuncSetAttribute(xrow_kernel<T, SCHEME, ONE, true>(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowSmemMax);
         if (dev >= 0 && dev < 64) attr_set[dev] = true;
     }
 }
@@ -141,42 +169,50 @@ static void launch_update_tma(BatchDev& b, dim3 g, double dt_scale, int final_st
     b.launches += 1;
 }
 
-// Update of one stage: the TMA-fed kernel for a single box whose rows are
-// whole 128-cell tiles, the z-column kernel otherwise.  A table launches both:
+// Update of one stage.  FP32: the pair kernel for every box (at 512^3 2.55 ms
+// a launch, at 320^3 0.63, where the bulk-copy fed kernel took 2.60 and, with
+// 64-cell tiles, 1.12).  FP64: the TMA-fed kernel for a single box whose rows
+// are whole 128-cell tiles, the z-column kernel otherwise.  A table launches both:
 // the z-column kernel skips the boxes with such rows (every box of a table is
 // carved on 256-byte boundaries), the TMA-fed kernel covers only those.
 template <class T, bool ONE>
 static void launch_update(BatchDev& b, double dt_scale, int final_stage) {
-    const dim3 gz = grid_of<ONE>(b, kKindCellZ);
-    // the bulk copies need 16-byte aligned sources: every row of a 128-cell
-    // tile starts on one when the field bases do
-    const bool aligned = ((uintptr_t)b.a.one.S[0] | (uintptr_t)b.a.one.F | (uintptr_t)b.a.one.E) % 16 == 0;
-    const int tw = tma_row_tile(b.a.one.nx, b.a.one.ny);
-    if (ONE && aligned && tw > 0) {
-        ensure_update_tma_attr<T>();
-        const dim3 g((unsigned)(b.a.one.nx / tw), (unsigned)(b.a.one.ny / (kTmaTile / tw)),
-                     (unsigned)ceil_shift(b.a.one.nz, b.a.one.segzs));
-        if (tw == kTmaTile) launch_update_tma<T, ONE, kTmaTile>(b, g, dt_scale, final_stage);
-        else launch_update_tma<T, ONE, kTmaTile / 2>(b, g, dt_scale, final_stage);
-        return;
-    }
-    if constexpr (ONE) {
-        if (short_columns<ONE>(b)) {
-            if (b.any_zrange) k_update<T, ONE, true, true><<<gz, kBX, 0, b.st>>>(b.a, dt_scale, final_stage);
-            else k_update<T, ONE, false, true><<<gz, kBX, 0, b.st>>>(b.a, dt_scale, final_stage);
-            b.launches += 1;
+    const dim3 gz = zgrid<T, ONE>(b);
+    if constexpr (sizeof(T) == 4) {
+        if (b.any_zrange) k_update_f32<ONE, true><<<gz, kBX, 0, b.st>>>(b.a, dt_scale, final_stage);
+        else k_update_f32<ONE, false><<<gz, kBX, 0, b.st>>>(b.a, dt_scale, final_stage);
+        b.launches += 1;
+    } else {
+        // the bulk copies need 16-byte aligned sources: every row of a 128-cell
+        // tile starts on one when the field bases do
+        const bool aligned = ((uintptr_t)b.a.one.S[0] | (uintptr_t)b.a.one.F | (uintptr_t)b.a.one.E) % 16 == 0;
+        const int tw = tma_row_tile(b.a.one.nx, b.a.one.ny);
+        if (ONE && aligned && tw > 0) {
+            ensure_update_tma_attr<T>();
+            const dim3 g((unsigned)(b.a.one.nx / tw), (unsigned)(b.a.one.ny / (kTmaTile / tw)),
+                         (unsigned)ceil_shift(b.a.one.nz, b.a.one.segzs));
+            if (tw == kTmaTile) launch_update_tma<T, ONE, kTmaTile>(b, g, dt_scale, final_stage);
+            else launch_update_tma<T, ONE, kTmaTile / 2>(b, g, dt_scale, final_stage);
             return;
         }
-    }
-    if (b.any_zrange) k_update<T, ONE, true><<<gz, kBX, 0, b.st>>>(b.a, dt_scale, final_stage);
-    else k_update<T, ONE, false><<<gz, kBX, 0, b.st>>>(b.a, dt_scale, final_stage);
-    b.launches += 1;
-    if (!ONE && (b.totals[kKindUpdTma] > 0 || b.totals[kKindUpdTma64] > 0)) {
-        ensure_update_tma_attr<T>();
-        if (b.totals[kKindUpdTma] > 0)
-            launch_update_tma<T, ONE, kTmaTile>(b, dim3((unsigned)b.totals[kKindUpdTma]), dt_scale, final_stage);
-        if (b.totals[kKindUpdTma64] > 0)
-            launch_update_tma<T, ONE, kTmaTile / 2>(b, dim3((unsigned)b.totals[kKindUpdTma64]), dt_scale, final_stage);
+        if constexpr (ONE) {
+            if (short_columns<ONE>(b)) {
+                if (b.any_zrange) k_update<T, ONE, true, true><<<gz, kBX, 0, b.st>>>(b.a, dt_scale, final_stage);
+                else k_update<T, ONE, false, true><<<gz, kBX, 0, b.st>>>(b.a, dt_scale, final_stage);
+                b.launches += 1;
+                return;
+            }
+        }
+        if (b.any_zrange) k_update<T, ONE, true><<<gz, kBX, 0, b.st>>>(b.a, dt_scale, final_stage);
+        else k_update<T, ONE, false><<<gz, kBX, 0, b.st>>>(b.a, dt_scale, final_stage);
+        b.launches += 1;
+        if (!ONE && (b.totals[kKindUpdTma] > 0 || b.totals[kKindUpdTma64] > 0)) {
+            ensure_update_tma_attr<T>();
+            if (b.totals[kKindUpdTma] > 0)
+                launch_update_tma<T, ONE, kTmaTile>(b, dim3((unsigned)b.totals[kKindUpdTma]), dt_scale, final_stage);
+            if (b.totals[kKindUpdTma64] > 0)
+                launch_update_tma<T, ONE, kTmaTile / 2>(b, dim3((unsigned)b.totals[kKindUpdTma64]), dt_scale, final_stage);
+        }
     }
 }
 
@@ -218,74 +254,95 @@ static void ensure_passive_pred_tma_attr() {
     }
 }
 
-// Passive predictor: the bulk-copy fed kernel for a single box whose rows are
-// whole 128-cell tiles (16-byte aligned sources), the z-column kernel
-// otherwise; scalar arrays sized for the table's largest passive count.
+// Passive predictor.  FP32: the pair kernel for every box (two scalars at 512^3
+// 0.78 ms, corrector 1.95, where the bulk-copy fed kernels took 1.20 and 2.05;
+// four at 320^3 0.36 and 0.92 against 0.58 and 1.43 of the z-column kernels).
+// FP64: the bulk-copy fed kernel for a single box whose rows are whole
+// 128-cell tiles (16-byte aligned sources), the z-column kernel otherwise;
+// scalar arrays sized for the table's largest passive count.
 template <class T, bool ONE>
 static void launch_passive_pred(BatchDev& b, dim3 gz) {
     const BoxRec& r = b.a.one;
-    if (ONE && ((uintptr_t)r.S[0] | (uintptr_t)r.SH) % 16 == 0 && passive_by_tma(r.nx)) {
-        ensure_passive_pred_tma_attr<T>();
-        const dim3 g((unsigned)(r.nx / kTmaTile), (unsigned)r.ny, (unsigned)ceil_shift(r.nz, r.segzs));
-        if (b.npass_max <= 2)
-            k_passive_pred_tma<T, 2><<<g, kTmaTile, passive_pred_tma_smem_bytes<T, 2>(), b.st>>>(b.a);
-        else if (b.npass_max <= 4)
-            k_passive_pred_tma<T, 4><<<g, kTmaTile, passive_pred_tma_smem_bytes<T, 4>(), b.st>>>(b.a);
-        else
-            k_passive_pred_tma<T, kMaxPass><<<g, kTmaTile, passive_pred_tma_smem_bytes<T, kMaxPass>(), b.st>>>(b.a);
+    if constexpr (sizeof(T) == 4) {
+        if (b.npass_max <= 1) k_passive_pred_f32<ONE, 1><<<gz, kBX, 0, b.st>>>(b.a);
+        else if (b.npass_max <= 2) k_passive_pred_f32<ONE, 2><<<gz, kBX, 0, b.st>>>(b.a);
+        else if (b.npass_max <= 4) k_passive_pred_f32<ONE, 4><<<gz, kBX, 0, b.st>>>(b.a);
+        else k_passive_pred_f32<ONE, kMaxPass><<<gz, kBX, 0, b.st>>>(b.a);
         b.launches += 1;
-        return;
-    }
-    if constexpr (ONE) {
-        if (short_columns<ONE>(b)) {
-            if (b.npass_max <= 2) k_passive_pred<T, ONE, 2, true><<<gz, kBX, 0, b.st>>>(b.a);
-            else if (b.npass_max <= 4) k_passive_pred<T, ONE, 4, true><<<gz, kBX, 0, b.st>>>(b.a);
-            else k_passive_pred<T, ONE, kMaxPass, true><<<gz, kBX, 0, b.st>>>(b.a);
+    } else {
+        if (ONE && ((uintptr_t)r.S[0] | (uintptr_t)r.SH) % 16 == 0 && passive_by_tma(r.nx)) {
+            ensure_passive_pred_tma_attr<T>();
+            const dim3 g((unsigned)(r.nx / kTmaTile), (unsigned)r.ny, (unsigned)ceil_shift(r.nz, r.segzs));
+            if (b.npass_max <= 2)
+                k_passive_pred_tma<T, 2><<<g, kTmaTile, passive_pred_tma_smem_bytes<T, 2>(), b.st>>>(b.a);
+            else if (b.npass_max <= 4)
+                k_passive_pred_tma<T, 4><<<g, kTmaTile, passive_pred_tma_smem_bytes<T, 4>(), b.st>>>(b.a);
+            else
+                k_passive_pred_tma<T, kMaxPass><<<g, kTmaTile, passive_pred_tma_smem_bytes<T, kMaxPass>(), b.st>>>(b.a);
             b.launches += 1;
             return;
         }
+        if constexpr (ONE) {
+            if (short_columns<ONE>(b)) {
+                if (b.npass_max <= 2) k_passive_pred<T, ONE, 2, true><<<gz, kBX, 0, b.st>>>(b.a);
+                else if (b.npass_max <= 4) k_passive_pred<T, ONE, 4, true><<<gz, kBX, 0, b.st>>>(b.a);
+                else k_passive_pred<T, ONE, kMaxPass, true><<<gz, kBX, 0, b.st>>>(b.a);
+                b.launches += 1;
+                return;
+            }
+        }
+        if (b.npass_max <= 2) k_passive_pred<T, ONE, 2><<<gz, kBX, 0, b.st>>>(b.a);
+        else if (b.npass_max <= 4) k_passive_pred<T, ONE, 4><<<gz, kBX, 0, b.st>>>(b.a);
+        else k_passive_pred<T, ONE, kMaxPass><<<gz, kBX, 0, b.st>>>(b.a);
+        b.launches += 1;
     }
-    if (b.npass_max <= 2) k_passive_pred<T, ONE, 2><<<gz, kBX, 0, b.st>>>(b.a);
-    else if (b.npass_max <= 4) k_passive_pred<T, ONE, 4><<<gz, kBX, 0, b.st>>>(b.a);
-    else k_passive_pred<T, ONE, kMaxPass><<<gz, kBX, 0, b.st>>>(b.a);
-    b.launches += 1;
 }
 
 template <class T, bool ONE>
 static void launch_passive_corr(BatchDev& b, dim3 gz) {
     const BoxRec& r = b.a.one;
-    if (ONE && ((uintptr_t)r.S[0] | (uintptr_t)r.SH | (uintptr_t)r.F) % 16 == 0 && passive_by_tma(r.nx)) {
-        ensure_passive_tma_attr<T>();
-        const dim3 g((unsigned)(r.nx / kTmaTile), (unsigned)r.ny, (unsigned)ceil_shift(r.nz, r.segzs));
-        if (b.npass_max <= 2)
-            k_passive_corr_tma<T, 2><<<g, kTmaTile, passive_tma_smem_bytes<T, 2>(), b.st>>>(b.a);
-        else if (b.npass_max <= 4)
-            k_passive_corr_tma<T, 4><<<g, kTmaTile, passive_tma_smem_bytes<T, 4>(), b.st>>>(b.a);
-        else
-            k_passive_corr_tma<T, kMaxPass><<<g, kTmaTile, passive_tma_smem_bytes<T, kMaxPass>(), b.st>>>(b.a);
+    if constexpr (sizeof(T) == 4) {
+        if (b.npass_max <= 1) k_passive_corr_f32<ONE, 1><<<gz, kBX, 0, b.st>>>(b.a);
+        else if (b.npass_max <= 2) k_passive_corr_f32<ONE, 2><<<gz, kBX, 0, b.st>>>(b.a);
+        else if (b.npass_max <= 4) k_passive_corr_f32<ONE, 4><<<gz, kBX, 0, b.st>>>(b.a);
+        else k_passive_corr_f32<ONE, kMaxPass><<<gz, kBX, 0, b.st>>>(b.a);
         b.launches += 1;
-        return;
-    }
-    if constexpr (ONE) {
-        if (short_columns<ONE>(b)) {
-            if (b.npass_max <= 2) k_passive_corr<T, ONE, 2, true><<<gz, kBX, 0, b.st>>>(b.a);
-            else if (b.npass_max <= 4) k_passive_corr<T, ONE, 4, true><<<gz, kBX, 0, b.st>>>(b.a);
-            else k_passive_corr<T, ONE, kMaxPass, true><<<gz, kBX, 0, b.st>>>(b.a);
+    } else {
+        if (ONE && ((uintptr_t)r.S[0] | (uintptr_t)r.SH | (uintptr_t)r.F) % 16 == 0 && passive_by_tma(r.nx)) {
+            ensure_passive_tma_attr<T>();
+            const dim3 g((unsigned)(r.nx / kTmaTile), (unsigned)r.ny, (unsigned)ceil_shift(r.nz, r.segzs));
+            if (b.npass_max <= 2)
+                k_passive_corr_tma<T, 2><<<g, kTmaTile, passive_tma_smem_bytes<T, 2>(), b.st>>>(b.a);
+            else if (b.npass_max <= 4)
+                k_passive_corr_tma<T, 4><<<g, kTmaTile, passive_tma_smem_bytes<T, 4>(), b.st>>>(b.a);
+            else
+                k_passive_corr_tma<T, kMaxPass><<<g, kTmaTile, passive_tma_smem_bytes<T, kMaxPass>(), b.st>>>(b.a);
             b.launches += 1;
             return;
         }
+        if constexpr (ONE) {
+            if (short_columns<ONE>(b)) {
+                if (b.npass_max <= 2) k_passive_corr<T, ONE, 2, true><<<gz, kBX, 0, b.st>>>(b.a);
+                else if (b.npass_max <= 4) k_passive_corr<T, ONE, 4, true><<<gz, kBX, 0, b.st>>>(b.a);
+                else k_passive_corr<T, ONE, kMaxPass, true><<<gz, kBX, 0, b.st>>>(b.a);
+                b.launches += 1;
+                return;
+            }
+        }
+        if (b.npass_max <= 2) k_passive_corr<T, ONE, 2><<<gz, kBX, 0, b.st>>>(b.a);
+        else if (b.npass_max <= 4) k_passive_corr<T, ONE, 4><<<gz, kBX, 0, b.st>>>(b.a);
+        else k_passive_corr<T, ONE, kMaxPass><<<gz, kBX, 0, b.st>>>(b.a);
+        b.launches += 1;
     }
-    if (b.npass_max <= 2) k_passive_corr<T, ONE, 2><<<gz, kBX, 0, b.st>>>(b.a);
-    else if (b.npass_max <= 4) k_passive_corr<T, ONE, 4><<<gz, kBX, 0, b.st>>>(b.a);
-    else k_passive_corr<T, ONE, kMaxPass><<<gz, kBX, 0, b.st>>>(b.a);
-    b.launches += 1;
 }
 
 template <class T>
 cudaError_t prepare_launch(BatchDev& b) {
-    ensure_update_tma_attr<T>();
-    ensure_passive_tma_attr<T>();
-    ensure_passive_pred_tma_attr<T>();
+    if constexpr (sizeof(T) == 8) {
+        ensure_update_tma_attr<T>();
+        ensure_passive_tma_attr<T>();
+        ensure_passive_pred_tma_attr<T>();
+    }
     for_schemes([&](auto s) {
         if (b.has_scheme[s.value]) {
             ensure_xrow_attr<T, s.value, true>();
@@ -298,17 +355,25 @@ cudaError_t prepare_launch(BatchDev& b) {
 template <class T, int SCHEME, bool ONE>
 static void launch_fluxes_corr_x(BatchDev& b) {
     if (!b.has_scheme[SCHEME]) return;
-    if (b.totals[scheme_kind(SCHEME, kSubXRow)]) {
-        dim3 gr = grid_of<ONE>(b, scheme_kind(SCHEME, kSubXRow));
-        size_t smem = 13 * (size_t)b.row_nx_max * sizeof(T);
+    const int krow = scheme_kind(SCHEME, kSubXRow), ktile = scheme_kind(SCHEME, kSubXTile);
+    if (b.totals[krow]) {
+        const bool pairs = b.row_pairs && pair_sweep<T, SCHEME, ONE>();
+        const dim3 gr = grid_of<ONE>(b, krow, pairs);
+        const size_t smem = 13 * (size_t)b.row_nx_max * sizeof(T) * (pairs ? 2 : 1);
         ensure_xrow_attr<T, SCHEME, ONE>();
-        int bd = b.row_nx_max >= 128 ? 128 : ((b.row_nx_max + 31) / 32) * 32;
-        k_corr_flux_xrow<T, SCHEME, ONE><<<gr, bd, smem, b.st>>>(b.a);
+        const int bd = b.row_nx_max >= 128 ? 128 : ((b.row_nx_max + 31) / 32) * 32;
+        if constexpr (pair_sweep<T, SCHEME, ONE>()) {
+            if (pairs) xrow_kernel<T, SCHEME, ONE, true>()<<<gr, bd, smem, b.st>>>(b.a);
+            else xrow_kernel<T, SCHEME, ONE, false>()<<<gr, bd, smem, b.st>>>(b.a);
+        } else {
+            xrow_kernel<T, SCHEME, ONE, false>()<<<gr, bd, smem, b.st>>>(b.a);
+        }
         b.launches += 1;
     }
-    if (b.totals[scheme_kind(SCHEME, kSubXTile)]) {
-        dim3 gt = grid_of<ONE>(b, scheme_kind(SCHEME, kSubXTile));
-        k_corr_flux_x<T, SCHEME, kTX, ONE><<<gt, kTX, 0, b.st>>>(b.a);
+    if (b.totals[ktile]) {
+        const dim3 gt = grid_of<ONE>(b, ktile);
+        if constexpr (pair_scheme<T, SCHEME, ONE>()) k_xtile_f32<SCHEME, kTX, ONE><<<gt, kTX, 0, b.st>>>(b.a);
+        else k_corr_flux_x<T, SCHEME, kTX, ONE><<<gt, kTX, 0, b.st>>>(b.a);
         b.launches += 1;
     }
 }
@@ -317,8 +382,9 @@ template <class T, int SCHEME, int D, bool ONE>
 static void launch_fluxes_corr_march(BatchDev& b) {
     const int kind = scheme_kind(SCHEME, D == 1 ? kSubMarchY : kSubMarchZ);
     if (!b.has_scheme[SCHEME] || b.totals[kind] == 0) return;
-    dim3 g = grid_of<ONE>(b, kind);
-    k_corr_flux_march<T, SCHEME, D, ONE><<<g, kBX, 0, b.st>>>(b.a);
+    const dim3 g = grid_of<ONE>(b, kind, pair_sweep<T, SCHEME, ONE>());
+    if constexpr (pair_scheme<T, SCHEME, ONE>()) k_sweep_f32<SCHEME, D, ONE><<<g, kBX, 0, b.st>>>(b.a);
+    else k_corr_flux_march<T, SCHEME, D, ONE><<<g, kBX, 0, b.st>>>(b.a);
     b.launches += 1;
 }
 
@@ -345,7 +411,7 @@ static void launch_protection(BatchDev& b, double dt_scale, int stage) {
 template <class T, bool ONE>
 static cudaError_t run_step_t(BatchDev& b, int device_driven) {
     const dim3 gc = grid_of<ONE>(b, kKindCell);
-    const dim3 gz = grid_of<ONE>(b, kKindCellZ);
+    const dim3 gz = zgrid<T, ONE>(b);
     const int nfin = (b.a.nbox + 31) / 32;
     b.prof_mask = 0;
     if (device_driven) {

@@ -5,9 +5,9 @@
 // operation (left-to-right evaluation, x**2 as x*x, SIGN as copysign, MAX/MIN
 // as `b > a ? b : a`), so that the FP64 instantiation, compiled with
 // --fmad=false and IEEE div/sqrt, reproduces a faithful CPU restatement bit
-// for bit.  The FP32 instantiation keeps the same formulas (with FMA
-// contraction) and evaluates the Roe / primitive eigenvector normalisation in
-// FP64 when the fast, slow and Alfven speeds are nearly degenerate.
+// for bit.  FP32 evaluates the rearranged forms of imhd_physics_fast.cuh; it
+// takes from here the FP64 eigenvector normalisations (where the fast, slow and
+// Alfven speeds are nearly degenerate), the PPM edges and the limiters.
 //
 // Rotated interface states use the reference's qint order
 // (vanleer_mod.f90:443-461): 0 rho, 1 m_n, 2 m_t1, 3 m_t2, 4 B_n, 5 B_t1, 6 B_t2.

@@ -1,17 +1,21 @@
 // imhd_physics_fast.cuh -- FP32 evaluation of the Riemann fluxes and of the
-// characteristic PLM slope.
+// characteristic slope, on one interface or cell (F1) or on two at once (F2).
 //
 // Same mathematics as imhd_physics.cuh (which keeps the reference's
 // operation order for the FP64 parity path), rearranged to issue fewer
 // instructions:
-//  * divisions by a density become one reciprocal and products, 1/sqrt
-//    becomes rsqrtf;
+//  * the states come as primitives and momenta, so that a velocity is divided
+//    out once per cell and never again per face;
+//  * divisions become one reciprocal and products, roots a reciprocal root;
+//  * the jumps enter as dm - v drho, which both families of a pair share;
 //  * the +/- eigenvector pairs of the fast, slow and Alfven families share
 //    their terms: L.d is formed as P +/- Q, R.dm from the sums and
 //    differences of the paired amplitudes;
 //  * the continuity sign flips of the Roe eigenvectors (K98 eq. 2.20) are
 //    dropped: they multiply both a left and the matching right eigenvector,
-//    so they cancel in the dissipation term.
+//    so they cancel in the dissipation term;
+//  * the limiter is homogeneous, so the constant factors of the left
+//    eigenvectors are applied once, after it;
 //  * the eigenvector renormalisation constants come from forms without
 //    cancellation: cs^2 = a^2 ca^2 / cf^2, the larger of cf^2 - ca^2 and
 //    cf^2 - a^2 as a sum of positive terms and the smaller from their
@@ -20,410 +24,366 @@
 #pragma once
 
 #include "imhd_physics.cuh"
+#include "imhd_value.cuh"
 
 namespace imhd {
 
+constexpr float kHalfRoot = 0.70710678118654752f;
+
+// One side of an interface in the rotated frame: density, velocity (n, t1,
+// t2), transverse field, momentum.
+template <class V>
+struct Side {
+    V r, v[3], b[2], m[3];
+};
+
+// Flux components: rho, m_n, m_t1, m_t2, B_t1, B_t2 (the six of a sweep's
+// flux fields, in their order).
+//
 // Roe flux of one interface (vanleer_mod.f90:2264-2863), FP32.
-__device__ __forceinline__ void flux_roe_fast(const float* uL, const float* uR, float cs, float asqr, float* Fo,
-                                              float& smax) {
-    float iL = 1.0f / uL[0], iR = 1.0f / uR[0];
-    float vxL = uL[1] * iL, vyL = uL[2] * iL, vzL = uL[3] * iL;
-    float vxR = uR[1] * iR, vyR = uR[2] * iR, vzR = uR[3] * iR;
-    float rho2 = 0.5f * (uL[0] + uR[0]);
-    float isrho = rsqrtf(rho2);
-    float srho = rho2 * isrho;
-    float vx2 = 0.5f * (vxL + vxR), vy2 = 0.5f * (vyL + vyR), vz2 = 0.5f * (vzL + vzR);
-    float Bx = uL[4];
-    float qa5 = Bx * isrho;
-    float qa6 = 0.5f * (uL[5] + uR[5]) * isrho;
-    float qa7 = 0.5f * (uL[6] + uR[6]) * isrho;
-    float btsqr = qa6 * qa6 + qa7 * qa7;
-    float ca2 = qa5 * qa5;
-    float bsqr = ca2 + btsqr;
-    float tmp1 = asqr + bsqr;
-    float dac = asqr - ca2;
-    float dd = dac - btsqr;
-    float tmp2 = sqrtf(dd * dd + 4.0f * asqr * btsqr);     // cf^2 - cs^2
-    float cf2 = 0.5f * (tmp1 + tmp2);
-    float icf = rsqrtf(cf2);
-    float ca = fabsf(qa5), cf = cf2 * icf;
-    float css = cs * ca * icf;                             // cf^2 cs^2 = a^2 ca^2
-    float ev0 = vx2 - cf, ev1 = vx2 - ca, ev2 = vx2 - css, ev3 = vx2 + css, ev4 = vx2 + ca, ev5 = vx2 + cf;
-    smax = fmaxf(smax, fabsf(vx2) + cf);
+template <class V>
+__device__ __forceinline__ void flux_roe_fast(const Side<V>& L, const Side<V>& R, V bn, float cs, float asqr, V* F,
+                                              V& smax) {
+    const V half = same<V>(0.5f), a1 = same<V>(cs), a2 = same<V>(asqr);
+    const V sr = L.r + R.r, sx = L.v[0] + R.v[0], sy = L.v[1] + R.v[1], sz = L.v[2] + R.v[2];
+    const V sb = L.b[0] + R.b[0], sc = L.b[1] + R.b[1];
+    const V rho = half * sr, vx = half * sx, vy = half * sy, vz = half * sz;
+    const V isr = vrsqrt(rho), srho = rho * isr, hisr = half * isr;
+    const V qx = bn * isr, qy = sb * hisr, qz = sc * hisr;
+    const V bt = fma(qy, qy, qz * qz), ca2 = qx * qx, dac = a2 - ca2, dd = dac - bt;
+    const V t2 = vsqrt(fma(dd, dd, same<V>(4.0f * asqr) * bt));          // cf^2 - cs^2
+    const V btt = bt + t2;
+    const V cf2 = half * ((a2 + ca2) + btt), icf = vrsqrt(cf2), cf = cf2 * icf;
+    const V ca = vabs(qx), css = (a1 * ca) * icf;                        // cf^2 cs^2 = a^2 ca^2
+    smax = vmax2(smax, vabs(vx) + cf);
 
-    float af, as;
-    if (tmp2 < 1.0e-2f * cf2) {
-        double afd, asd;
-        roe_alphas_fp64((double)qa5, (double)qa6, (double)qa7, (double)asqr, afd, asd);
-        af = (float)afd;
-        as = (float)asd;
-    } else {
-        // af = sqrt(cf^2 - ca^2) / sqrt(cf^2 - cs^2), as = sqrt(cf^2 - a^2) / sqrt(cf^2 - cs^2): the
-        // larger radicand is big, the smaller cf^2 bt^2 / big
-        float big = 0.5f * (fabsf(dac) + btsqr + tmp2);
-        float q = rsqrtf(big * tmp2);
-        float cfbt = cf * sqrtf(btsqr);
-        af = (dac >= 0.0f ? big : cfbt) * q;
-        as = (dac >= 0.0f ? cfbt : big) * q;
+    // af = sqrt(cf^2 - ca^2) / sqrt(cf^2 - cs^2), as = sqrt(cf^2 - a^2) / sqrt(cf^2 - cs^2): the larger
+    // radicand is big, the smaller cf^2 bt^2 / big; no transverse field: beta = (1, 1) / sqrt 2
+    const V big = half * (vabs(dac) + btt), q = vrsqrt(big * t2);
+    const V ib = each([](float b) { return b < 1.0e-30f ? 0.0f : rsqrtf(b); }, bt);
+    const V cfbt = cf * (bt * ib);
+    V af = vsel(dac, big, cfbt) * q, as = vsel(dac, cfbt, big) * q;
+    if (any_less(t2, same<V>(1.0e-2f) * cf2)) {
+#pragma unroll 1
+        for (int l = 0; l < lanes_of<V>::n; ++l) {
+            if (lane(t2, l) < 1.0e-2f * lane(cf2, l)) {
+                double afd, asd;
+                roe_alphas_fp64((double)lane(qx, l), (double)lane(qy, l), (double)lane(qz, l), (double)asqr, afd, asd);
+                set_lane(af, l, (float)afd);
+                set_lane(as, l, (float)asd);
+            }
+        }
     }
-    float gy, gz;
-    if (btsqr < 1.0e-30f) {
-        gy = 0.70710678118654752f;
-        gz = 0.70710678118654752f;
-    } else {
-        float ib = rsqrtf(btsqr);
-        gy = qa6 * ib;
-        gz = qa7 * ib;
-    }
-    float signbx = copysignf(1.0f, qa5);
+    const V gy = each([](float i, float g) { return i == 0.0f ? kHalfRoot : g; }, ib, qy * ib);
+    const V gz = each([](float i, float g) { return i == 0.0f ? kHalfRoot : g; }, ib, qz * ib);
+    const V ngy = same<V>(-1.0f) * gy;
+    const V S = vsign(1.0f, qx);
 
-    // characteristic amplitudes (K98 eq. 2.16-2.19, 2.27)
-    float dq0 = uR[0] - uL[0], dq1 = uR[1] - uL[1], dq2 = uR[2] - uL[2], dq3 = uR[3] - uL[3];
-    float dq4 = uR[5] - uL[5], dq5 = uR[6] - uL[6];
-    float af2 = af * af, as2 = as * as;
-    float it1 = 0.5f / (af2 * asqr + as2 * cf2);
-    float it2 = 0.5f / (af2 * cs * cf + as2 * css * ca);
-    float vt = gy * vy2 + gz * vz2;
-    float dqt = gy * dq2 + gz * dq3;    // transverse momentum jump along beta
-    float dbt = gy * dq4 + gz * dq5;    // transverse field jump along beta
-    // fast
-    float t1 = it1 * af * asqr;
-    float t2 = it2 * (as * css * signbx * vt - af * cs * vx2);
-    float t3 = it2 * as * css * signbx;
-    float t4 = it1 * as * cf * srho;
-    float Pf = dq0 * t1 + t4 * dbt;
-    float Qf = t3 * dqt - dq0 * t2 - dq1 * (it2 * af * cs);
-    float ck0 = Pf + Qf, ck5 = Pf - Qf;
-    // Alfven
-    float Ua = 0.5f * signbx * ((gz * dq2 - gy * dq3) - dq0 * (gz * vy2 - gy * vz2));
-    float Va = 0.5f * srho * (gz * dq4 - gy * dq5);
-    float ck1 = Ua + Va, ck4 = Va - Ua;
-    // slow
-    float s1 = it1 * as * cf2;
-    float s2 = it2 * (as * ca * vx2 + af * cf * signbx * vt);
-    float s3 = it2 * af * cf * signbx;
-    float s4 = it1 * af * cf * srho;
-    float Ps = dq0 * s1 - s4 * dbt;
-    float Qs = dq0 * s2 - dq1 * (it2 * as * ca) - s3 * dqt;
-    float ck2 = Ps + Qs, ck3 = Ps - Qs;
+    // characteristic amplitudes (K98 eq. 2.16-2.19, 2.27), the 1/2 of the flux average included
+    const V d0 = R.r - L.r, nd0 = L.r - R.r;
+    const V wn = fma(vx, nd0, R.m[0] - L.m[0]), w2 = fma(vy, nd0, R.m[1] - L.m[1]), w3 = fma(vz, nd0, R.m[2] - L.m[2]);
+    const V e2 = R.b[0] - L.b[0], e3 = R.b[1] - L.b[1];
+    const V wt = fma(gy, w2, gz * w3), wa = fma(gz, w2, ngy * w3);
+    const V et = fma(gy, e2, gz * e3), ea = fma(gz, e2, ngy * e3);
+    const V afc = af * a1, afcf = af * cf, asc = as * css, asca = as * ca, ascf = as * cf;
+    const V quarter = same<V>(0.25f);
+    const V i1 = quarter * vrcp(fma(afc, afc, ascf * ascf)), i2 = quarter * vrcp(fma(afc, afcf, asc * asca));
+    const V X = srho * et, Sw = S * wt;
+    const V Pf = i1 * fma(ascf, X, (afc * a1) * d0);
+    const V Ps = i1 * ((ascf * cf) * d0 - afcf * X);
+    const V Qf = i2 * (asc * Sw - afc * wn);
+    const V Qs = i2 * fma(asca, wn, afcf * Sw);        // with the sign turned
+    const V U = S * wa, W = srho * ea;                 // Alfven amplitudes without their 1/2 (in h below)
 
-    // Harten entropy fix, delta = 0.3 on the fast and slow families (vanleer_mod.f90:78, 2829-2833)
-    auto harten = [](float ev, float c) {
-        float a = fabsf(ev);
-        return (a >= 0.3f ? a : (a + 0.09f) * (1.0f / 0.6f)) * c;
+    // -|ev| c with Harten's entropy fix, delta = 0.3, on the fast and slow families
+    // (vanleer_mod.f90:78, 2829-2833)
+    auto harten = [](V ev, V c) {
+        return each([](float e) {
+                   const float a = -fabsf(e);
+                   return a <= -0.3f ? a : __fmul_rn(__fadd_rn(a, -0.09f), 1.0f / 0.6f);
+               }, ev) * c;
     };
-    float b0 = harten(ev0, ck0), b5 = harten(ev5, ck5);
-    float b2 = harten(ev2, ck2), b3 = harten(ev3, ck3);
-    float b1 = fabsf(ev1) * ck1, b4 = fabsf(ev4) * ck4;
+    auto nabs = [](V ev) { return each([](float e) { return -fabsf(e); }, ev); };
+    const V b0 = harten(vx - cf, Pf + Qf), b5 = harten(vx + cf, Pf - Qf);
+    const V b2 = harten(vx - css, Ps - Qs), b3 = harten(vx + css, Ps + Qs);
+    const V b1 = nabs(vx - ca) * (U + W), b4 = nabs(vx + ca) * (W - U);
 
-    // sum_k beta_k R_k with the right eigenvectors of K98 eq. 2.12
-    float sF = b0 + b5, dF = b0 - b5;
-    float sA = b1 + b4, dA = b1 - b4;
-    float sS = b2 + b3, dS = b3 - b2;
-    float t5f = as * cf * isrho;
-    float t5s = af * asqr * isrho * icf;
-    float dis0 = af * sF + as * sS;
-    float dis1 = af * (b0 * ev0 + b5 * ev5) + as * (b2 * ev2 + b3 * ev3);
-    float q2 = as * qa5 * dF + af * cs * signbx * dS;      // coefficient of beta in components 2, 3
-    float dis2 = vy2 * (af * sF + as * sS) + gy * q2 + signbx * gz * dA;
-    float dis3 = vz2 * (af * sF + as * sS) + gz * q2 - signbx * gy * dA;
-    float c4 = t5f * sF - t5s * sS;
-    float dis4 = gy * c4 + isrho * gz * sA;
-    float dis5 = gz * c4 - isrho * gy * sA;
+    // minus sum_k beta_k R_k with the right eigenvectors of K98 eq. 2.12
+    const V sF = b0 + b5, dF = b0 - b5, sS = b2 + b3, dS = b3 - b2, sA = b1 + b4, dA = b1 - b4;
+    const V m = fma(af, sF, as * sS);
+    const V q2 = S * fma(asca, dF, afc * dS);
+    const V hA = (quarter * isr) * sA, SA = vsign(0.25f, qx) * dA;
+    const V c4 = isr * (ascf * sF - (afc * (a1 * icf)) * sS);
+    const V n1 = fma(vx, m, asc * dS - afcf * dF);
+    const V n2 = fma(vy, m, fma(gy, q2, gz * SA)), n3 = fma(vz, m, fma(gz, q2, ngy * SA));
+    const V n4 = fma(gy, c4, gz * hA), n5 = fma(gz, c4, ngy * hA);
 
-    // physical fluxes (vanleer_mod.f90:2765-2801)
-    float hb = 0.5f * (uL[5] * uL[5] + uL[6] * uL[6] - Bx * Bx);
-    float hbR = 0.5f * (uR[5] * uR[5] + uR[6] * uR[6] - Bx * Bx);
-    float FL0 = uL[1], FR0 = uR[1];
-    float FL1 = uL[1] * vxL + uL[0] * asqr + hb;
-    float FR1 = uR[1] * vxR + uR[0] * asqr + hbR;
-    float FL2 = uL[1] * vyL - Bx * uL[5], FR2 = uR[1] * vyR - Bx * uR[5];
-    float FL3 = uL[1] * vzL - Bx * uL[6], FR3 = uR[1] * vzR - Bx * uR[6];
-    float FL4 = vxL * uL[5] - vyL * Bx, FR4 = vxR * uR[5] - vyR * Bx;
-    float FL5 = vxL * uL[6] - vzL * Bx, FR5 = vxR * uR[6] - vzR * Bx;
-    Fo[0] = 0.5f * (FL0 + FR0 - dis0);
-    Fo[1] = 0.5f * (FL1 + FR1 - dis1);
-    Fo[2] = 0.5f * (FL2 + FR2 - dis2);
-    Fo[3] = 0.5f * (FL3 + FR3 - dis3);
-    Fo[4] = 0.0f;
-    Fo[5] = 0.5f * (FL4 + FR4 - dis4);
-    Fo[6] = 0.5f * (FL5 + FR5 - dis5);
+    // plus the mean of the physical fluxes (vanleer_mod.f90:2765-2801)
+    const V nb = same<V>(-1.0f) * bn;
+    const V bb = fma(L.b[0], L.b[0], fma(L.b[1], L.b[1], fma(R.b[0], R.b[0], R.b[1] * R.b[1])));
+    const V pr = fma(a2, sr, fma(half, bb, bn * nb));
+    F[0] = fma(half, L.m[0] + R.m[0], m);
+    F[1] = fma(half, fma(L.m[0], L.v[0], fma(R.m[0], R.v[0], pr)), n1);
+    F[2] = fma(half, fma(L.m[0], L.v[1], fma(R.m[0], R.v[1], nb * sb)), n2);
+    F[3] = fma(half, fma(L.m[0], L.v[2], fma(R.m[0], R.v[2], nb * sc)), n3);
+    F[4] = fma(half, fma(L.v[0], L.b[0], fma(R.v[0], R.b[0], nb * sy)), n4);
+    F[5] = fma(half, fma(L.v[0], L.b[1], fma(R.v[0], R.b[1], nb * sz)), n5);
 }
 
-// Fast magnetosonic speed of a conserved rotated state given 1/rho.
-__device__ __forceinline__ float fast_speed_fast(const float* u, float irho, float asqr) {
-    float btsqr = (u[5] * u[5] + u[6] * u[6]) * irho;
-    float bsqr = u[4] * u[4] * irho + btsqr;
-    float tmp1 = asqr + bsqr, dd = asqr - bsqr;
-    float tmp2 = sqrtf(dd * dd + 4.0f * asqr * btsqr);
-    return sqrtf(0.5f * (tmp1 + tmp2));
+// Fast magnetosonic speed given 1/rho, B_n^2 and the transverse field squared.
+template <class V>
+__device__ __forceinline__ V fast_speed_fast(V ir, V bn2, V bt2, float asqr) {
+    const V bt = bt2 * ir, s = fma(bn2, ir, bt), a2 = same<V>(asqr), dd = a2 - s;
+    const V t2 = vsqrt(fma(dd, dd, same<V>(4.0f * asqr) * bt));
+    return vsqrt(same<V>(0.5f) * ((a2 + s) + t2));
 }
 
-__device__ __forceinline__ void phys_flux_fast(const float* u, float vx, float vy, float vz, float asqr, float* F) {
-    F[0] = u[1];
-    F[1] = u[1] * vx + u[0] * asqr + 0.5f * (u[5] * u[5] + u[6] * u[6] - u[4] * u[4]);
-    F[2] = u[1] * vy - u[4] * u[5];
-    F[3] = u[1] * vz - u[4] * u[6];
-    F[4] = 0.0f;
-    F[5] = vx * u[5] - vy * u[4];
-    F[6] = vx * u[6] - vz * u[4];
+// Signal speeds of HLLE and HLLD (vanleer_mod.f90:2895-2962, 3020-3086).
+template <class V>
+__device__ __forceinline__ void hll_speeds(const Side<V>& L, const Side<V>& R, V bn, float asqr, V& sL, V& sR, V& smax) {
+    const V half = same<V>(0.5f), zero = same<V>(0.0f), bn2 = bn * bn;
+    const V ia = vrcp(half * (L.r + R.r)), vxa = (half * (L.m[0] + R.m[0])) * ia;
+    const V ab = half * (L.b[0] + R.b[0]), ac = half * (L.b[1] + R.b[1]);
+    const V cL = fast_speed_fast(vrcp(L.r), bn2, fma(L.b[0], L.b[0], L.b[1] * L.b[1]), asqr);
+    const V cR = fast_speed_fast(vrcp(R.r), bn2, fma(R.b[0], R.b[0], R.b[1] * R.b[1]), asqr);
+    const V cm = fast_speed_fast(ia, bn2, fma(ab, ab, ac * ac), asqr);
+    sL = vmin2(vmin2(L.v[0] - cL, vxa - cm), zero);
+    sR = vmax2(vmax2(R.v[0] + cR, vxa + cm), zero);
+    smax = vmax2(vmax2(smax, vabs(L.v[0]) + cL), vmax2(vabs(R.v[0]) + cR, vabs(vxa) + cm));
+}
+
+template <class V>
+__device__ __forceinline__ void phys_flux_fast(const Side<V>& s, V bn, V nb, float asqr, V* F) {
+    const V bt = fma(s.b[0], s.b[0], fma(s.b[1], s.b[1], bn * nb));
+    F[0] = s.m[0];
+    F[1] = fma(s.m[0], s.v[0], fma(same<V>(asqr), s.r, same<V>(0.5f) * bt));
+    F[2] = fma(s.m[0], s.v[1], nb * s.b[0]);
+    F[3] = fma(s.m[0], s.v[2], nb * s.b[1]);
+    F[4] = fma(s.v[0], s.b[0], nb * s.v[1]);
+    F[5] = fma(s.v[0], s.b[1], nb * s.v[2]);
 }
 
 // HLLE flux (vanleer_mod.f90:2867-2981), FP32.
-__device__ __forceinline__ void flux_hlle_fast(const float* uL, const float* uR, float asqr, float* Fo, float& smax) {
-    float iL = 1.0f / uL[0], iR = 1.0f / uR[0];
-    float vxL = uL[1] * iL, vyL = uL[2] * iL, vzL = uL[3] * iL;
-    float vxR = uR[1] * iR, vyR = uR[2] * iR, vzR = uR[3] * iR;
-    float ua[7];
+template <class V>
+__device__ __forceinline__ void flux_hlle_fast(const Side<V>& L, const Side<V>& R, V bn, float asqr, V* F, V& smax) {
+    V sL, sR, FL[6], FR[6];
+    hll_speeds(L, R, bn, asqr, sL, sR, smax);
+    const V nb = same<V>(-1.0f) * bn;
+    phys_flux_fast(L, bn, nb, asqr, FL);
+    phys_flux_fast(R, bn, nb, asqr, FR);
+    const V is = vrcp(sR - sL), x = sR * is, y = (same<V>(-1.0f) * sL) * is, z = sL * x;
+    const V du[6] = {R.r - L.r, R.m[0] - L.m[0], R.m[1] - L.m[1], R.m[2] - L.m[2], R.b[0] - L.b[0], R.b[1] - L.b[1]};
 #pragma unroll
-    for (int m = 0; m < 7; ++m) ua[m] = 0.5f * (uL[m] + uR[m]);
-    float ia = 1.0f / ua[0];
-    float FL[7], FR[7];
-    phys_flux_fast(uL, vxL, vyL, vzL, asqr, FL);
-    phys_flux_fast(uR, vxR, vyR, vzR, asqr, FR);
-    float cfL = fast_speed_fast(uL, iL, asqr), cfR = fast_speed_fast(uR, iR, asqr), cfa = fast_speed_fast(ua, ia, asqr);
-    float vxa = ua[1] * ia;
-    float sL = fminf(fminf(vxL - cfL, vxa - cfa), 0.0f);
-    float sR = fmaxf(fmaxf(vxR + cfR, vxa + cfa), 0.0f);
-    smax = fmaxf(fmaxf(fmaxf(smax, fabsf(vxL) + cfL), fabsf(vxR) + cfR), fabsf(vxa) + cfa);
-    float isRL = 1.0f / (sR - sL);
-    float sRsL = sR * sL;
-#pragma unroll
-    for (int m = 0; m < 7; ++m) Fo[m] = (sR * FL[m] - sL * FR[m] + sRsL * (uR[m] - uL[m])) * isRL;
+    for (int c = 0; c < 6; ++c) F[c] = fma(x, FL[c], fma(y, FR[c], z * du[c]));
 }
 
-// Isothermal HLLD flux (Mignone 2007; vanleer_mod.f90:2986-3239), FP32.
-__device__ __forceinline__ void flux_hlld_fast(const float* uL, const float* uR, float asqr, float* Fo, float& smax) {
-    const float ZERO = 1.0e-20f;
-    float iL = 1.0f / uL[0], iR = 1.0f / uR[0];
-    float Bx = uL[4];
-    float vxL = uL[1] * iL, vyL = uL[2] * iL, vzL = uL[3] * iL;
-    float vxR = uR[1] * iR, vyR = uR[2] * iR, vzR = uR[3] * iR;
-    float ua[7];
+// Isothermal HLLD flux (Mignone 2007; vanleer_mod.f90:2986-3239), FP32.  Every
+// star region is evaluated and the one of the interface selected; density and
+// normal momentum take the HLL flux in all of them (F_K + s_K (U_hll - U_K)
+// is the HLL flux), and the supersonic cases take the flux of one side.
+template <class V>
+__device__ __forceinline__ void flux_hlld_fast(const Side<V>& L, const Side<V>& R, V bn, float asqr, V* F, V& smax) {
+    V sL, sR, FL[6], FR[6];
+    hll_speeds(L, R, bn, asqr, sL, sR, smax);
+    const V half = same<V>(0.5f), nb = same<V>(-1.0f) * bn, bn2 = bn * bn;
+    phys_flux_fast(L, bn, nb, asqr, FL);
+    phys_flux_fast(R, bn, nb, asqr, FR);
+    const V is = vrcp(sR - sL), z = sR * sL;
+    const V rs = ((sR * R.r - sL * L.r) - (FR[0] - FL[0])) * is;
+    F[0] = fma(z, R.r - L.r, sR * FL[0] - sL * FR[0]) * is;
+    F[1] = fma(z, R.m[0] - L.m[0], sR * FL[1] - sL * FR[1]) * is;
+    const V irs = vrcp(rs), isr = vrsqrt(rs), vs = F[0] * irs, ax = vabs(bn) * isr;
+    const V aL = vs - ax, aR = vs + ax;
+    // star state of one side: m_t1, m_t2, B_t1, B_t2; the side's own where its
+    // outer wave meets an Alfven wave
+    auto star = [&](const Side<V>& u, V s, V* o) {
+        const V xl = s - aL, xr = s - aR;
+        const V i = vrcp(xl * xr), dv = s - u.v[0];
+        const V t1 = (bn * (vs - u.v[0])) * i, t2 = ((u.r * dv) * dv - bn2) * (irs * i);
+        const V near = vmin2(vabs(xl), vabs(xr)) - same<V>(1.0e-20f);
+        o[0] = vsel(near, rs * u.v[1] - t1 * u.b[0], u.m[1]);
+        o[1] = vsel(near, rs * u.v[2] - t1 * u.b[1], u.m[2]);
+        o[2] = vsel(near, t2 * u.b[0], u.b[0]);
+        o[3] = vsel(near, t2 * u.b[1], u.b[1]);
+    };
+    V uL[4], uR[4];
+    star(L, sL, uL);
+    star(R, sR, uR);
+    const V srs = rs * isr, S = vsign(1.0f, bn), X = srs * S, iX = isr * S, nbi = nb * irs;
+    const V naR = same<V>(-1.0f) * aR;
 #pragma unroll
-    for (int m = 0; m < 7; ++m) ua[m] = 0.5f * (uL[m] + uR[m]);
-    float ia = 1.0f / ua[0];
-    float FL[7], FR[7];
-    phys_flux_fast(uL, vxL, vyL, vzL, asqr, FL);
-    phys_flux_fast(uR, vxR, vyR, vzR, asqr, FR);
-    float cfL = fast_speed_fast(uL, iL, asqr), cfR = fast_speed_fast(uR, iR, asqr), cfa = fast_speed_fast(ua, ia, asqr);
-    float vxa = ua[1] * ia;
-    float sL = fminf(fminf(vxL - cfL, vxa - cfa), 0.0f);
-    float sR = fmaxf(fmaxf(vxR + cfR, vxa + cfa), 0.0f);
-    smax = fmaxf(fmaxf(fmaxf(smax, fabsf(vxL) + cfL), fabsf(vxR) + cfR), fabsf(vxa) + cfa);
-    if (sL >= 0.0f) {
-#pragma unroll
-        for (int m = 0; m < 7; ++m) Fo[m] = FL[m];
-        return;
+    for (int c = 0; c < 2; ++c) {
+        const V um = half * fma(X, uR[2 + c] - uL[2 + c], uL[c] + uR[c]);
+        const V ub = half * fma(iX, uR[c] - uL[c], uL[2 + c] + uR[2 + c]);
+        const V fm = fma(um, vs, nb * ub), fb = fma(vs, ub, um * nbi);
+        F[2 + c] = vsel(aL, fma(sL, uL[c] - L.m[1 + c], FL[2 + c]),
+                        vsel(naR, fma(sR, uR[c] - R.m[1 + c], FR[2 + c]), fm));
+        F[4 + c] = vsel(aL, fma(sL, uL[2 + c] - L.b[c], FL[4 + c]),
+                        vsel(naR, fma(sR, uR[2 + c] - R.b[c], FR[4 + c]), fb));
     }
-    if (sR <= 0.0f) {
+    // sL = 0: everything leaves to the right; sR = 0: to the left
+    if (any_less(vmin2(sR, same<V>(-1.0f) * sL), same<V>(1.0e-37f))) {
+        const V nsR = same<V>(-1.0f) * sR;
 #pragma unroll
-        for (int m = 0; m < 7; ++m) Fo[m] = FR[m];
-        return;
+        for (int c = 0; c < 6; ++c) F[c] = vsel(sL, FL[c], vsel(nsR, FR[c], F[c]));
     }
-    float isRL = 1.0f / (sR - sL);
-    float sRsL = sR * sL;
-    float rho_s = (sR * uR[0] - sL * uL[0] - FR[0] + FL[0]) * isRL;
-    float momx_s = (sR * uR[1] - sL * uL[1] - FR[1] + FL[1]) * isRL;
-    float FHLL0 = (sR * FL[0] - sL * FR[0] + sRsL * (uR[0] - uL[0])) * isRL;
-    float FHLL1 = (sR * FL[1] - sL * FR[1] + sRsL * (uR[1] - uL[1])) * isRL;
-    float irho_s = 1.0f / rho_s;
-    float vx_s = FHLL0 * irho_s;
-    float isrho_s = rsqrtf(rho_s);
-    float abx = fabsf(Bx) * isrho_s;
-    float sLs = vx_s - abx, sRs = vx_s + abx;
-    float uLs[7], uRs[7];
-    uLs[0] = rho_s; uLs[1] = momx_s;
-    if ((fabsf(sL - sLs) < ZERO) || (fabsf(sL - sRs) < ZERO)) {
-#pragma unroll
-        for (int m = 2; m < 7; ++m) uLs[m] = uL[m];
-    } else {
-        float is = 1.0f / ((sL - sLs) * (sL - sRs));
-        float t1 = Bx * (vx_s - vxL) * is;
-        float dv = sL - vxL;
-        float t2 = (uL[0] * dv * dv - Bx * Bx) * irho_s * is;
-        uLs[2] = rho_s * vyL - t1 * uL[5];
-        uLs[3] = rho_s * vzL - t1 * uL[6];
-        uLs[4] = uL[4];
-        uLs[5] = t2 * uL[5];
-        uLs[6] = t2 * uL[6];
-    }
-    uRs[0] = rho_s; uRs[1] = momx_s;
-    if ((fabsf(sR - sLs) < ZERO) || (fabsf(sR - sRs) < ZERO)) {
-#pragma unroll
-        for (int m = 2; m < 7; ++m) uRs[m] = uR[m];
-    } else {
-        float is = 1.0f / ((sR - sLs) * (sR - sRs));
-        float t1 = Bx * (vx_s - vxR) * is;
-        float dv = sR - vxR;
-        float t2 = (uR[0] * dv * dv - Bx * Bx) * irho_s * is;
-        uRs[2] = rho_s * vyR - t1 * uR[5];
-        uRs[3] = rho_s * vzR - t1 * uR[6];
-        uRs[4] = uR[4];
-        uRs[5] = t2 * uR[5];
-        uRs[6] = t2 * uR[6];
-    }
-    if (sLs >= 0.0f) {
-#pragma unroll
-        for (int m = 0; m < 7; ++m) Fo[m] = FL[m] + sL * (uLs[m] - uL[m]);
-    } else if (sRs <= 0.0f) {
-#pragma unroll
-        for (int m = 0; m < 7; ++m) Fo[m] = FR[m] + sR * (uRs[m] - uR[m]);
-    } else {
-        float srs = rho_s * isrho_s;    // sqrt(rho_s)
-        float X = copysignf(srs, Bx);
-        float iX = copysignf(isrho_s, Bx);
-        float uC2 = 0.5f * (uLs[2] + uRs[2] + X * (uRs[5] - uLs[5]));
-        float uC3 = 0.5f * (uLs[3] + uRs[3] + X * (uRs[6] - uLs[6]));
-        float uC5 = 0.5f * (uLs[5] + uRs[5] + iX * (uRs[2] - uLs[2]));
-        float uC6 = 0.5f * (uLs[6] + uRs[6] + iX * (uRs[3] - uLs[3]));
-        Fo[0] = FHLL0;
-        Fo[1] = FHLL1;
-        Fo[2] = uC2 * vx_s - Bx * uC5;
-        Fo[3] = uC3 * vx_s - Bx * uC6;
-        Fo[4] = 0.0f;
-        Fo[5] = vx_s * uC5 - uC2 * Bx * irho_s;
-        Fo[6] = vx_s * uC6 - uC3 * Bx * irho_s;
-    }
+}
+
+// Monotonised-central limiter times two, without its 1/2 and with the factor
+// beta = 1.01 on the one-sided differences (mc_limit): the least of 2 beta dL,
+// 2 beta dR and dL + dR where all are positive, the largest where all are
+// negative, otherwise 0.
+template <class V>
+__device__ __forceinline__ V mc_twice(V dl, V dr) {
+    const V k = same<V>((float)(2.0 * kMC_BETA));
+    const V x = k * dl, y = k * dr, c = dl + dr;
+    const V lo = vmin2(vmin2(x, y), c), hi = vmax2(vmax2(x, y), c);
+    return each([](float a) { return fmaxf(a, 0.0f); }, lo) + each([](float a) { return fminf(a, 0.0f); }, hi);
 }
 
 // Limited characteristic slope of one cell (S08 A12/A22, vanleer_mod.f90:
 // 941-1141, 1507-1546), FP32.  wm, w0, wp: rotated primitives of cells
 // i-1, i, i+1; bn: face field at i+1/2.
-template <bool PPM = false>
-__device__ __forceinline__ void plm_char_slope_fast(const float* wm, const float* w0, const float* wp,
-                                                    const float* wp2, float bn, float cs, float asqr, float* delw) {
-    float rho = w0[0];
-    float irho = 1.0f / rho;
-    float irhos = rsqrtf(rho);
-    float rhos = rho * irhos;
-    float bx = irhos * bn, by = irhos * w0[4], bz = irhos * w0[5];
-    float btsqr = by * by + bz * bz;
-    float ca2 = bx * bx;
-    float bsqr = ca2 + btsqr;
-    float tmp1 = asqr + bsqr;
-    float dac = asqr - ca2;
-    float dd = dac - btsqr;
-    float tmp2 = sqrtf(dd * dd + 4.0f * asqr * btsqr);     // cf^2 - cs^2
-    float cf2 = 0.5f * (tmp1 + tmp2);
-    float icf = rsqrtf(cf2);
-    float cf = cf2 * icf;
-    float css = cs * fabsf(bx) * icf;                      // cf^2 cs^2 = a^2 ca^2
-    float af, as;
-    if (tmp2 < 1.0e-2f * cf2) {
-        double afd, asd;
-        prim_alphas_fp64<float>((double)rho, (double)bn, (double)w0[4], (double)w0[5], (double)asqr, afd, asd);
-        af = (float)afd;
-        as = (float)asd;
-    } else {
-        // af^2 = (a^2 - cs^2) / tmp2 = a^2 (cf^2 - ca^2) / (cf^2 tmp2), as^2 = (cf^2 - a^2) / tmp2; the
-        // larger of cf^2 - ca^2 and cf^2 - a^2 is big, the smaller cf^2 bt^2 / big
-        float big = 0.5f * (fabsf(dac) + btsqr + tmp2);
-        float bt = sqrtf(btsqr);
-        if (dac >= 0.0f) {
-            float q = rsqrtf(cf2 * tmp2 * big);
-            af = cs * big * q;
-            as = cf2 * bt * q;
-        } else {
-            float q = rsqrtf(tmp2 * big);
-            af = cs * bt * q;
-            as = big * q;
+template <bool PPM, class V>
+__device__ __forceinline__ void plm_char_slope_fast(const V* wm, const V* w0, const V* wp, const V* wp2, V bn, float cs,
+                                                    float asqr, V* delw) {
+    const V half = same<V>(0.5f), a1 = same<V>(cs), a2 = same<V>(asqr);
+    const V rho = w0[0], irs = vrsqrt(rho), rhos = rho * irs;
+    const V bx = irs * bn, by = irs * w0[4], bz = irs * w0[5];
+    const V bt = fma(by, by, bz * bz), ca2 = bx * bx, dac = a2 - ca2, dd = dac - bt;
+    const V t2 = vsqrt(fma(dd, dd, same<V>(4.0f * asqr) * bt));          // cf^2 - cs^2
+    const V btt = bt + t2;
+    const V cf2 = half * ((a2 + ca2) + btt), icf = vrsqrt(cf2), cf = cf2 * icf;
+    const V css = (a1 * vabs(bx)) * icf;                                 // cf^2 cs^2 = a^2 ca^2
+    // af^2 = (a^2 - cs^2) / t2 = a^2 (cf^2 - ca^2) / (cf^2 t2), as^2 = (cf^2 - a^2) / t2; the larger of
+    // cf^2 - ca^2 and cf^2 - a^2 is big, the smaller cf^2 bt^2 / big
+    const V big = half * (vabs(dac) + btt), q = vrsqrt(big * t2);
+    const V ib = each([](float b) { return b < 1.0e-30f ? 0.0f : rsqrtf(b); }, bt);
+    const V sb = bt * ib;
+    V af = (a1 * q) * vsel(dac, big * icf, sb), as = q * vsel(dac, cf * sb, big);
+    if (any_less(t2, same<V>(1.0e-2f) * cf2)) {
+#pragma unroll 1
+        for (int l = 0; l < lanes_of<V>::n; ++l) {
+            if (lane(t2, l) < 1.0e-2f * lane(cf2, l)) {
+                double afd, asd;
+                prim_alphas_fp64<float>((double)lane(rho, l), (double)lane(bn, l), (double)lane(w0[4], l),
+                                        (double)lane(w0[5], l), (double)asqr, afd, asd);
+                set_lane(af, l, (float)afd);
+                set_lane(as, l, (float)asd);
+            }
         }
     }
-    float gy, gz;
-    if (btsqr < 1.0e-30f) {
-        gy = 0.70710678118654752f;
-        gz = 0.70710678118654752f;
-    } else {
-        float ib = rsqrtf(btsqr);
-        gy = by * ib;
-        gz = bz * ib;
+    const V gy = each([](float i, float g) { return i == 0.0f ? kHalfRoot : g; }, ib, by * ib);
+    const V gz = each([](float i, float g) { return i == 0.0f ? kHalfRoot : g; }, ib, bz * ib);
+    const V ngz = same<V>(-1.0f) * gz, naf = same<V>(-1.0f) * af;
+    const V S = vsign(1.0f, bx);
+    const V Cf = cf * af, Cs = css * as, Qf = Cf * S, Qs = Cs * S;
+    const V k0 = (a2 * irs) * irs, k1 = a1 * irs, Si = S * irs;
+    // left eigenvectors (S08 A22) times the differences, without the factors
+    // 1/(2 a^2) (fast, slow) and 1/2 (Alfven)
+    constexpr int NS = PPM ? 3 : 2;   // projected differences: w0-wm, wp-w0 (, wp2-wp)
+    V aD[NS][6];
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+        V d[6];
+#pragma unroll
+        for (int m = 0; m < 6; ++m) d[m] = s == 0 ? w0[m] - wm[m] : s == 1 ? wp[m] - w0[m] : wp2[m] - wp[m];
+        V* a = aD[s];
+        const V dvt = fma(gy, d[2], gz * d[3]), dbt = fma(gy, d[4], gz * d[5]);
+        const V p0 = k0 * d[0], p1 = k1 * dbt;
+        const V P = fma(af, p0, as * p1), Q = Qs * dvt - Cf * d[1];
+        const V P2 = fma(as, p0, naf * p1), Q2 = fma(Cs, d[1], Qf * dvt);   // Q2 with the sign turned
+        const V U = fma(gy, d[3], ngz * d[2]), W = Si * fma(gy, d[5], ngz * d[4]);
+        a[0] = P + Q;
+        a[5] = P - Q;
+        a[2] = P2 - Q2;
+        a[3] = P2 + Q2;
+        a[1] = U + W;
+        a[4] = W - U;
     }
-    float S = copysignf(1.0f, bx);
-    float Nf = 0.5f / asqr;
-    // left-eigenvector coefficients (S08 A22)
-    float f0 = 0.5f * af * irho, f1 = Nf * cf * af, fq = Nf * css * as * S, fa = Nf * cs * as * irhos;
-    float s0 = 0.5f * as * irho, s1 = Nf * css * as, sq_ = Nf * cf * af * S, sa = Nf * cs * af * irhos;
-    float hS = 0.5f * S * irhos;
-    float dm[6];
-    {
-        constexpr int NS = PPM ? 3 : 2;   // projected differences: w0-wm, wp-w0 (, wp2-wp)
-        float dD[NS][6];
+    V dm[6];
 #pragma unroll
-        for (int m = 0; m < 6; ++m) {
-            dD[0][m] = w0[m] - wm[m];
-            dD[1][m] = wp[m] - w0[m];
-            if constexpr (PPM) dD[2][m] = wp2[m] - wp[m];
-        }
-        float aD[NS][6];
-#pragma unroll
-        for (int s = 0; s < NS; ++s) {
-            const float* d = dD[s];
-            float* a = aD[s];
-            float dvt = gy * d[2] + gz * d[3];
-            float dbt = gy * d[4] + gz * d[5];
-            float P = f0 * d[0] + fa * dbt, Q = fq * dvt - f1 * d[1];
-            a[0] = P + Q; a[5] = P - Q;
-            float P2 = s0 * d[0] - sa * dbt, Q2 = -s1 * d[1] - sq_ * dvt;
-            a[2] = P2 + Q2; a[3] = P2 - Q2;
-            float U = 0.5f * (gy * d[3] - gz * d[2]), V = hS * (gy * d[5] - gz * d[4]);
-            a[1] = U + V; a[4] = V - U;
-        }
-#pragma unroll
-        for (int k = 0; k < 6; ++k) {
-            float m1 = mc_limit(aD[0][k], aD[1][k], 0.5f * (aD[0][k] + aD[1][k]));
-            if constexpr (PPM) dm[k] = mc_limit(aD[1][k], aD[2][k], 0.5f * (aD[1][k] + aD[2][k])) - m1;
-            else dm[k] = m1;
-        }
+    for (int k = 0; k < 6; ++k) {
+        dm[k] = mc_twice(aD[0][k], aD[1][k]);
+        if constexpr (PPM) dm[k] = mc_twice(aD[1][k], aD[2][k]) - dm[k];
     }
-    // right eigenvectors (S08 A12) applied to the limited amplitudes
-    float sf = dm[0] + dm[5], df = dm[5] - dm[0];
-    float ss = dm[2] + dm[3], ds = dm[3] - dm[2];
-    float sA = dm[1] + dm[4], dA = dm[4] - dm[1];
-    float Qs = css * as * S, Qf = cf * af * S, As = cs * as * rhos, Af = cs * af * rhos;
-    float tq = Qf * ds - Qs * df;
-    float ta = As * sf - Af * ss;
-    float Srh = S * rhos;
-    delw[0] = rho * (af * sf + as * ss);
-    delw[1] = cf * af * df + css * as * ds;
-    delw[2] = gy * tq + gz * dA;
+    // right eigenvectors (S08 A12) applied to the limited amplitudes, with the
+    // factors left out above and the limiter's 1/2
+    const V kN = same<V>(0.25f / asqr), kA = same<V>(0.25f);
+    const V sf = kN * (dm[0] + dm[5]), df = kN * (dm[5] - dm[0]);
+    const V ss = kN * (dm[2] + dm[3]), ds = kN * (dm[3] - dm[2]);
+    const V sA = kA * (dm[1] + dm[4]), dA = kA * (dm[4] - dm[1]);
+    const V tq = Qf * ds - Qs * df;
+    const V ta = (a1 * rhos) * fma(as, sf, naf * ss);
+    const V SA = (S * rhos) * sA;
+    delw[0] = rho * fma(af, sf, as * ss);
+    delw[1] = fma(Cf, df, Cs * ds);
+    delw[2] = fma(gy, tq, gz * dA);
     delw[3] = gz * tq - gy * dA;
-    delw[4] = gy * ta - gz * Srh * sA;
-    delw[5] = gz * ta + gy * Srh * sA;
+    delw[4] = fma(gy, ta, ngz * SA);
+    delw[5] = fma(gz, ta, gy * SA);
 }
 
-}  // namespace imhd
-
-namespace imhd {
-
-// Precision dispatch: the FP64 path keeps the reference's operation order
-// (bit parity with the oracle), the FP32 path uses the rearranged forms above.
-template <int SOLVER, class T>
-__device__ __forceinline__ void riemann_flux(const T* uL, const T* uR, T cs, T asqr, T* Fo, T& smax) {
-    if constexpr (std::is_same<T, float>::value) {
-        if (SOLVER == 1 || SOLVER == 4) flux_roe_fast(uL, uR, cs, asqr, Fo, smax);
-        else if (SOLVER == 2) flux_hlld_fast(uL, uR, asqr, Fo, smax);
-        else flux_hlle_fast(uL, uR, asqr, Fo, smax);
-    } else {
-        riemann<SOLVER>(uL, uR, cs, asqr, Fo, smax);
+// Primitive-variable slopes (prim_slope), FP32.
+template <bool PPM, class V>
+__device__ __forceinline__ void prim_slope_fast(const V* wm, const V* w0, const V* wp, const V* wp2, V* delw) {
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+        if constexpr (PPM)
+            delw[k] = each([](float a, float b, float c) { return prim_ppm_limit(a, b, c); }, wm[k], w0[k], wp[k]) -
+                      each([](float a, float b, float c) { return prim_ppm_limit(a, b, c); }, w0[k], wp[k], wp2[k]);
+        else
+            delw[k] = each([](float a, float b, float c) {
+                const float dL = b - a, dR = c - b, dC = 0.5f * (dL + dR);
+                return sgn1(dC) * vmin(vmin((float)kMC_BETA * fabsf(dL), (float)kMC_BETA * fabsf(dR)), fabsf(dC));
+            }, wm[k], w0[k], wp[k]);
     }
 }
 
-template <class T, bool PPM = false>
-__device__ __forceinline__ void char_slope(const T* wm, const T* w0, const T* wp, const T* wp2, T bn, T cs, T asqr,
-                                           T* delw) {
-    if constexpr (std::is_same<T, float>::value) plm_char_slope_fast<PPM>(wm, w0, wp, wp2, bn, cs, asqr, delw);
-    else plm_char_slope<T, PPM>(wm, w0, wp, wp2, bn, cs, asqr, delw);
+template <int SOLVER, class V>
+__device__ __forceinline__ void riemann_fast(const Side<V>& L, const Side<V>& R, V bn, float cs, float asqr, V* F,
+                                             V& smax) {
+    if constexpr (SOLVER == 1 || SOLVER == 4) flux_roe_fast(L, R, bn, cs, asqr, F, smax);   // 4: with protection fluxes
+    else if constexpr (SOLVER == 2) flux_hlld_fast(L, R, bn, asqr, F, smax);
+    else flux_hlle_fast(L, R, bn, asqr, F, smax);
 }
 
 // Slope of a sweep's reconstruction (scheme_recon: bit 0 PPM, bit 1 primitive
 // variables): the characteristic slope or the primitive-variable one.
-template <class T, int RECON>
-__device__ __forceinline__ void recon_slope(const T* wm, const T* w0, const T* wp, const T* wp2, T bn, T cs, T asqr,
-                                           T* delw) {
+template <int RECON, class V>
+__device__ __forceinline__ void recon_slope_fast(const V* wm, const V* w0, const V* wp, const V* wp2, V bn, float cs,
+                                                 float asqr, V* delw) {
     constexpr bool PPM = (RECON & 1) != 0;
-    if constexpr ((RECON & 2) != 0) prim_slope<T, PPM>(wm, w0, wp, wp2, delw);
-    else char_slope<T, PPM>(wm, w0, wp, wp2, bn, cs, asqr, delw);
+    if constexpr ((RECON & 2) != 0) prim_slope_fast<PPM>(wm, w0, wp, wp2, delw);
+    else plm_char_slope_fast<PPM>(wm, w0, wp, wp2, bn, cs, asqr, delw);
+}
+
+// Interface side from a cell's primitives and a multiple h of its slope
+// (+1/2: the state left of its upper face, -1/2: right of its lower one), or
+// from a PPM edge.
+template <class V>
+__device__ __forceinline__ void side_of(const V* w, Side<V>& s) {
+    s.r = w[0];
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+        s.v[m] = w[1 + m];
+        s.m[m] = w[1 + m] * w[0];
+    }
+    s.b[0] = w[4];
+    s.b[1] = w[5];
+}
+// PPM edge values (ppm_edges) of F1 values.
+template <bool PRIM>
+__device__ __forceinline__ void ppm_edges_fast(const F1* wm, const F1* w0, const F1* wp, const F1* dm, const F1* d0,
+                                               F1* wl, F1* wr) {
+    ppm_edges<float, PRIM>(&wm->v, &w0->v, &wp->v, &dm->v, &d0->v, &wl->v, &wr->v);
+}
+template <class V>
+__device__ __forceinline__ void plm_side(const V* w, const V* d, float h, Side<V>& s) {
+    V e[6];
+#pragma unroll
+    for (int m = 0; m < 6; ++m) e[m] = fma(same<V>(h), d[m], w[m]);
+    side_of(e, s);
 }
 
 }  // namespace imhd

@@ -266,7 +266,7 @@ struct Worker {
             d.a.one = r.rec;
             d.a.one.active = 1;
             d.a.nbox = 1;
-            for (int k = 0; k < imhd::kKinds; ++k) d.totals[k] = (int)imhd::blocks_of(r.rec, k, s->esz);
+            for (int k = 0; k < imhd::kKinds; ++k) d.totals[k] = (int)imhd::blocks_of(r.rec, k, s->esz, false, true);
             d.st = bst;
             if (!bck(f64 ? imhd::run_max_speed<double>(d) : imhd::run_max_speed<float>(d), "initial CFL")) return false;
             imhd::Scalars back;

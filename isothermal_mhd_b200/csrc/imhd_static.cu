@@ -27,6 +27,7 @@
 //    across one.
 #include <cuda_runtime.h>
 
+#include <cstdint>
 #include <cstring>
 #include <mutex>
 #include <string>
@@ -109,6 +110,7 @@ extern "C" int imhd_step_static(int precision, int nx, int ny, int nz, int riema
     imhd::BoxRec rec;
     imhd::init_rec(rec, nx, ny, nz, npass, riemann, IMHD_PLM, sound_speed, cour, 0.0, 0.0);
     imhd::one_box_segments(rec, esz);
+    if (((uintptr_t)state_in | (uintptr_t)state_out) % 8) rec.vec = 0;   // no 8-byte accesses to the caller's rows
     rec.S[0] = const_cast<void*>(state_in);
     rec.S[1] = state_out;
     unsigned char* p = base;
@@ -125,7 +127,7 @@ extern "C" int imhd_step_static(int precision, int nx, int ny, int nz, int riema
     b.st = (cudaStream_t)stream;
     std::vector<imhd::BoxRec> recs(1, rec);
     std::vector<int> prefix;
-    if (!imhd::build_prefix(recs, esz, prefix, b)) return fail(IMHD_E_ARG, "box too large for one launch");
+    if (!imhd::build_prefix(recs, esz, prefix, b, true)) return fail(IMHD_E_ARG, "box too large for one launch");
     b.a.boxes = (imhd::BoxRec*)table;
     b.a.prefix = (const int*)(table + 256);
     b.a.use_one = 1;                                      // the box travels in the launch parameters

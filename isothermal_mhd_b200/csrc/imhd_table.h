@@ -21,13 +21,38 @@ inline int reduction_blocks(int n) {
     return b < kRedBlocksMax ? b : kRedBlocksMax;
 }
 
+// FP32 boxes take two interfaces per thread: pairs of cells in the predictor
+// and, with PLM (PPM's window is too large for two), in the y / z sweeps, pairs
+// of rows in the x sweep unless the longest row would then exceed the shared
+// memory of the x-row sweep.  The Roe boxes of a table keep one interface per
+// thread (imhd_physics_table.cuh).
+inline bool pair_fluxes(const BoxRec& r, size_t esz, bool single) { return esz == 4 && (single || r.riemann != 1); }
+inline bool pair_sweeps(const BoxRec& r, size_t esz, bool single) {
+    return pair_fluxes(r, esz, single) && !(r.recon & 1);
+}
+// Width (log2) of the x tiles of pairs: the one that leaves the fewest threads
+// idle, the widest among equals, no wider than the box's cell tiles.
+inline int pair_tile(int nx, int tws) {
+    int best = 4;
+    long least = 0;
+    for (int t = 4; t <= tws; ++t) {
+        const long used = (long)ceil_div(pairs_of(nx), 1 << t) << t;
+        if (t == 4 || used <= least) { best = t; least = used; }
+    }
+    return best;
+}
+
 // Blocks of box r for decomposition `kind`.
-inline long blocks_of(const BoxRec& r, int kind, size_t esz) {
+inline long blocks_of(const BoxRec& r, int kind, size_t esz, bool row_pairs, bool single) {
     const int tw = 1 << r.tws, th = kBX >> r.tws;
     long nbx = ceil_div(r.nx, tw), nby = ceil_div(r.ny, th), nbz = ceil_div(r.nz, th);
     if (kind == kKindCell) return nbx * nby * r.nz;
-    if (kind == kKindCellZ) return nbx * nby * ceil_div(r.nz, 1 << r.segzs);
+    if (kind == kKindCellZ) return esz == 4 ? 0 : nbx * nby * ceil_div(r.nz, 1 << r.segzs);
+    if (kind == kKindPairZ)
+        return esz == 4 ? (long)ceil_div(pairs_of(r.nx), 1 << r.ptws) * ceil_div(r.ny, kBX >> r.ptws) * ceil_div(r.nz, 1 << r.segzs)
+                        : 0;
     if (kind == kKindRed) return r.nred;
+    if (esz == 4 && (kind == kKindUpdTma || kind == kKindUpdTma64)) return 0;   // FP64 kernels
     if (kind == kKindUpdTma) return r.nx % kTmaTile == 0 ? (long)(r.nx / kTmaTile) * r.ny * ceil_div(r.nz, kSegZ) : 0;
     if (kind == kKindUpdTma64)
         return (r.nx % kTmaTile != 0 && r.nx % (kTmaTile / 2) == 0 && r.ny % 2 == 0)
@@ -37,9 +62,15 @@ inline long blocks_of(const BoxRec& r, int kind, size_t esz) {
     int sub = (kind - kKindSolver0) % 5;
     if (scheme_of(box_solver(r), r.recon) != scheme) return 0;
     bool row = row_capable(r.nx, esz);
+    const bool pairs = pair_sweeps(r, esz, single);
+    if (sub == kSubCell ? pair_fluxes(r, esz, single) : pairs) {
+        nbx = ceil_div(pairs_of(r.nx), 1 << r.ptws);
+        nby = ceil_div(r.ny, kBX >> r.ptws);
+        nbz = ceil_div(r.nz, kBX >> r.ptws);
+    }
     switch (sub) {
         case kSubCell: return nbx * nby * ceil_div(r.nz, 1 << r.segzs);   // z columns of the predictor fluxes
-        case kSubXRow: return row ? (long)r.ny * r.nz : 0;
+        case kSubXRow: return row ? (long)(row_pairs && pairs ? ceil_div(r.ny, 2) : r.ny) * r.nz : 0;
         case kSubXTile: return row ? 0 : (long)ceil_div(r.nx, kTX) * r.ny * r.nz;
         case kSubMarchY: return nbx * nbz * ceil_div(r.ny, 1 << r.segs);   // (x, z) tiles marching along y
         default: return nbx * nby * ceil_div(r.nz, 1 << r.segs);           // (x, y) tiles marching along z
@@ -48,8 +79,10 @@ inline long blocks_of(const BoxRec& r, int kind, size_t esz) {
 
 // Prefix sums of every kind (kKinds rows of nbox+1 ints) and the launch
 // parameters of the table.  Returns false when a launch would exceed the
-// 2^31-1 block limit of a grid.
-inline bool build_prefix(const std::vector<BoxRec>& recs, size_t esz, std::vector<int>& prefix, BatchDev& bd);
+// 2^31-1 block limit of a grid.  single: one box, launched by its own record
+// (use_one), not a table.
+inline bool build_prefix(const std::vector<BoxRec>& recs, size_t esz, std::vector<int>& prefix, BatchDev& bd,
+                         bool single);
 
 // Box of every block, per kind (for tables of more than one box).
 inline void build_blk2box(const std::vector<int>& prefix, int nbox, const BatchDev& bd,
@@ -64,20 +97,24 @@ inline void build_blk2box(const std::vector<int>& prefix, int nbox, const BatchD
     }
 }
 
-inline bool build_prefix(const std::vector<BoxRec>& recs, size_t esz, std::vector<int>& prefix, BatchDev& bd) {
+inline bool build_prefix(const std::vector<BoxRec>& recs, size_t esz, std::vector<int>& prefix, BatchDev& bd,
+                         bool single) {
     int nbox = (int)recs.size();
+    bd.row_nx_max = 0;
+    for (const BoxRec& r : recs)
+        if (row_capable(r.nx, esz) && r.nx > bd.row_nx_max) bd.row_nx_max = r.nx;
+    bd.row_pairs = esz == 4 && 2 * 13 * (size_t)bd.row_nx_max * esz <= kRowSmemMax;
     prefix.assign((size_t)kKinds * (nbox + 1), 0);
     for (int k = 0; k < kKinds; ++k) {
         long acc = 0;
         for (int b = 0; b < nbox; ++b) {
             prefix[(size_t)k * (nbox + 1) + b] = (int)acc;
-            acc += blocks_of(recs[b], k, esz);
+            acc += blocks_of(recs[b], k, esz, bd.row_pairs, single);
             if (acc > 2147483647L) return false;
         }
         prefix[(size_t)k * (nbox + 1) + nbox] = (int)acc;
         bd.totals[k] = (int)acc;
     }
-    bd.row_nx_max = 0;
     for (int s = 0; s <= kSchemes; ++s) bd.has_scheme[s] = false;
     bd.any_pass = false;
     bd.npass_max = 0;
@@ -90,7 +127,6 @@ inline bool build_prefix(const std::vector<BoxRec>& recs, size_t esz, std::vecto
         if (r.npass > 0) bd.any_pass = true;
         if (r.npass > bd.npass_max) bd.npass_max = r.npass;
         if (r.zlo != 0 || r.zhi != r.nz) bd.any_zrange = true;
-        if (row_capable(r.nx, esz) && r.nx > bd.row_nx_max) bd.row_nx_max = r.nx;
     }
     bd.a.nbox = nbox;
     return true;
@@ -105,7 +141,7 @@ struct TablePlan {
 };
 
 inline bool plan_table(const std::vector<BoxRec>& recs, size_t esz, BatchDev& bd, TablePlan& tp) {
-    if (!build_prefix(recs, esz, tp.prefix, bd)) return false;
+    if (!build_prefix(recs, esz, tp.prefix, bd, false)) return false;
     build_blk2box(tp.prefix, (int)recs.size(), bd, tp.b2b);
     tp.bytes = align256(sizeof(BoxRec) * recs.size()) + align256(tp.prefix.size() * sizeof(int));
     for (int k = 0; k < kKinds; ++k) tp.bytes += align256(tp.b2b[k].size() * sizeof(int) + 4);
@@ -169,6 +205,8 @@ inline void init_rec(BoxRec& r, int nx, int ny, int nz, int npass, int riemann, 
     // widest x tile that the row length divides (whole 128-byte segments per
     // warp, no idle threads), 32 when none does
     r.tws = (nx % 128 == 0) ? 7 : (nx % 64 == 0) ? 6 : 5;
+    r.ptws = (short)pair_tile(nx, r.tws);
+    r.vec = nx % 2 == 0;
     // y / z sweep segments: 32 faces per thread on long columns (measured at
     // 512^3: y 3.0 -> 2.9 ms, PPM 4.5 -> 4.3), 16 otherwise (more threads for
     // small boxes; batches tune this further)
@@ -210,13 +248,15 @@ inline double column_cost(long blocks_per_unit, int len, double start, int occ, 
 // 192^3 1827, 1932, 1987 (16 stays); FP64 64^3 577, 375, 385, 372, 393; 96^3
 // 1044, 953, 983, 1052, 1202; 128^3 2154, 2020, 2093; 192^3 7135, 7176.
 inline void one_box_segments(BoxRec& r, size_t esz) {
-    const int tw = 1 << r.tws, th = kBX >> r.tws, occ = esz == 8 ? 2 : 6, fill = esz == 8 ? 2 : 4;
-    const long nbx = ceil_div(r.nx, tw);
-    const long sweep = nbx * ((long)ceil_div(r.nz, th) * r.ny + (long)ceil_div(r.ny, th) * r.nz) / 2;
-    const long cols = nbx * ceil_div(r.ny, th) * r.nz;
+    const bool pairs = pair_sweeps(r, esz, true);
+    const int tws = pairs ? r.ptws : r.tws, nu = pairs ? pairs_of(r.nx) : r.nx, th = kBX >> tws;
+    const int occ = esz == 8 ? 2 : 6, fill = esz == 8 ? 2 : 4, socc = pairs ? 3 : occ, sfill = pairs ? 2 : fill;
+    const long sweep = ceil_div(nu, 1 << tws) *
+                       ((long)ceil_div(r.nz, th) * r.ny + (long)ceil_div(r.ny, th) * r.nz) / 2;
+    const long cols = (long)ceil_div(r.nx, 1 << r.tws) * ceil_div(r.ny, kBX >> r.tws) * r.nz;
     double best = 0.0;
     for (int s = 0; s <= 5; ++s) {
-        const double c = column_cost(sweep, 1 << s, 0.6, occ, fill);
+        const double c = column_cost(sweep, 1 << s, 0.6, socc, sfill);
         if (s == 0 || c <= best) { best = c; r.segs = s; }
     }
     if (cols < 8L * 148 * kSegZ) {

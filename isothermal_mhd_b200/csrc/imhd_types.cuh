@@ -35,7 +35,8 @@ enum Kind {
     kKindCellZ = 82,   // (x, y) tiles per z segment, a z column of kSegZ cells per thread
     kKindUpdTma = 83,  // 128-cell row segments per z segment of the bulk-copy fed update (rows of 128k cells)
     kKindUpdTma64 = 84,// pairs of 64-cell row segments per z segment of it (rows of 64(2k+1) cells, even ny)
-    kKinds = 85
+    kKindPairZ = 85,   // (x, y) tiles of cell pairs per z segment (FP32 boxes)
+    kKinds = 86
 };
 // A scheme is a flux solver (1 Roe, 2 HLLD, 3 HLLE, 4 Roe with the HLLE
 // protection fluxes beside it) with a reconstruction (0 PLM and 1 PPM of the
@@ -106,8 +107,11 @@ struct BoxRec {
     void* Ep;
     unsigned char* bad;
     int* badlist;
-    int badcap, pad3_;
+    int badcap;
+    short ptws, vec;    // FP32 pair sweeps: x tile of 1 << ptws cell pairs; the rows are whole aligned pairs
 };
+// x pairs of a row, for the FP32 sweeps that take two cells per thread.
+__host__ __device__ inline int pairs_of(int nx) { return (nx + 1) / 2; }
 // Flux solver of a box's scheme (4: Roe with protection fluxes).
 __host__ __device__ inline int box_solver(const BoxRec& r) { return (r.riemann == 1 && r.protect) ? 4 : r.riemann; }
 
@@ -130,6 +134,7 @@ struct BatchDev {
     int totals[kKinds];        // blocks per kind (grid sizes)
     int row_nx_max = 0;        // largest nx among boxes using the x-row sweep
     bool has_scheme[kSchemes + 1] = {};
+    bool row_pairs = false;    // the FP32 x-row sweep stages two rows per block
     bool any_pass = false;
     int npass_max = 0;         // largest passive count of the table
     bool any_zrange = false;   // some box restricts its maxima to a z range
