@@ -436,22 +436,19 @@ int imhd_step(imhd_box* x, double dt, int drive_next, double* dt_next) {
     if (!(dt > 0.0)) return fail(IMHD_E_ARG, "dt must be positive");
     if (drive_next && !x->have_force) return fail(IMHD_E_STATE, "drive step requested before imhd_set_force");
     CK(cudaSetDevice(x->cfg.device));
-    imhd::Scalars* sc = x->rec.sc;
-    x->hio[0] = dt;
-    int drive = drive_next ? 1 : 0;
-    std::memcpy(x->hio + 4, &drive, sizeof(int));
-    CK(cudaMemcpyAsync(&sc->dt, x->hio, sizeof(double), cudaMemcpyHostToDevice, x->b.st));
-    CK(cudaMemcpyAsync(&sc->drive, x->hio + 4, sizeof(int), cudaMemcpyHostToDevice, x->b.st));
-    x->b.drive_mode = drive;
+    x->b.drive_mode = drive_next ? 1 : 0;
+    x->rec.dt = dt;
+    x->rec.drive = x->b.drive_mode;
+    x->b.a.report = x->hio + 32;     // the last kernel of the step writes dt_next and the status here
     CK(step_dispatch(x));
     x->cur ^= 1;
-    CK(cudaMemcpyAsync(x->hio + 1, &sc->dt_next, sizeof(double), cudaMemcpyDeviceToHost, x->b.st));
-    CK(cudaMemcpyAsync((unsigned*)(x->hio + 2), &sc->status, sizeof(unsigned), cudaMemcpyDeviceToHost, x->b.st));
     int rc = sync_and_check(x);
     if (rc) return rc;
     if ((rc = accumulate_stage_times(x))) return rc;
-    if (dt_next) *dt_next = x->hio[1];
-    unsigned st = *(unsigned*)(x->hio + 2);
+    if (dt_next) *dt_next = x->hio[32];
+    long long bits;
+    std::memcpy(&bits, x->hio + 33, sizeof(bits));
+    const unsigned st = (unsigned)bits;
     if (st & IMHD_S_WAIT) return fail(IMHD_E_CUDA, "a bounded wait for an asynchronous copy gave up");
     if (st & IMHD_S_NAN) return fail(IMHD_E_PHYSICS, "non-finite state or max speed: the step is not valid");
     if (st & IMHD_S_ZERO_SPEED) return fail(IMHD_E_PHYSICS, "zero max speed encountered");

@@ -53,6 +53,24 @@ __device__ __forceinline__ BoxRec resolve(const BatchArgs& ba, int kind, int& lo
         return ba.boxes[b];
     }
 }
+// Start of a single box's step kernel: it may be scheduled while the kernel
+// before it in the step still runs (programmatic stream serialization, see
+// launch() in imhd_launch.cuh), and waits here until that one has completed and
+// its writes are visible; then the kernel after it may be scheduled.  Nothing
+// a kernel reads or writes comes before this call.  No-op where a launch does
+// not ask for it (tables, and kernels outside a step).
+template <bool ONE>
+__device__ __forceinline__ void step_enter() {
+    if constexpr (ONE) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    }
+}
+// This step's dt and drive flag.
+template <bool ONE>
+__device__ __forceinline__ double step_dt(const BoxRec& rp) { return ONE ? rp.dt : rp.sc->dt; }
+template <bool ONE>
+__device__ __forceinline__ int step_drive(const BoxRec& rp) { return ONE ? rp.drive : rp.sc->drive; }
 // Box b of the table (the kernels that run one thread or block per box).
 __device__ __forceinline__ BoxRec box_at(const BatchArgs& ba, int b) { return ba.use_one ? ba.one : ba.boxes[b]; }
 __device__ __forceinline__ Dims dims_of(const BoxRec& r) { return Dims{r.nx, r.ny, r.nz, r.n}; }
@@ -224,6 +242,7 @@ __device__ __forceinline__ void protection_flux(const T* uL, const T* uR, T cs, 
 template <class T, int SCHEME, bool ONE, bool SHORT = false>
 __global__ void __launch_bounds__(kBX, sizeof(T) == 4 ? 5 : 1)
 k_pred_flux(BatchArgs ba) {
+    step_enter<ONE>();
     constexpr int SOLVER = scheme_solver(SCHEME);
     int local;
     const BoxRec rp = resolve<ONE>(ba, scheme_kind(SCHEME, kSubCell), local);
@@ -328,6 +347,7 @@ __device__ __forceinline__ void store_flux(T* __restrict__ F, int D, int n, int 
 // k_sweep_f32.
 template <class T, int SCHEME, int D, bool ONE>
 __global__ void __launch_bounds__(kBX, sizeof(T) == 4 ? 6 : 1) k_corr_flux_march(BatchArgs ba) {
+    step_enter<ONE>();
     constexpr int SOLVER = scheme_solver(SCHEME);
     constexpr int RECON = scheme_recon(SCHEME);
     constexpr bool PPM = (RECON & 1) != 0, PRIM = (RECON & 2) != 0;
@@ -437,6 +457,7 @@ __global__ void __launch_bounds__(kBX, sizeof(T) == 4 ? 6 : 1) k_corr_flux_march
 // shared memory.
 template <class T, int SCHEME, int TX, bool ONE>
 __global__ void __launch_bounds__(TX) k_corr_flux_x(BatchArgs ba) {
+    step_enter<ONE>();
     constexpr int SOLVER = scheme_solver(SCHEME);
     constexpr int RECON = scheme_recon(SCHEME);
     constexpr bool PPM = (RECON & 1) != 0, PRIM = (RECON & 2) != 0;
@@ -532,6 +553,7 @@ __global__ void __launch_bounds__(TX) k_corr_flux_x(BatchArgs ba) {
 // 4.67 -> 4.58e9 cell-updates/s); other FP32 boxes run k_xrow_f32.
 template <class T, int SCHEME, bool ONE>
 __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 8 : 1) k_corr_flux_xrow(BatchArgs ba) {
+    step_enter<ONE>();
     constexpr int SOLVER = scheme_solver(SCHEME);
     constexpr int RECON = scheme_recon(SCHEME);
     constexpr bool PPM = (RECON & 1) != 0, PRIM = (RECON & 2) != 0;
@@ -797,6 +819,7 @@ __device__ __forceinline__ void pred_flux_f32(const BoxRec& rp, int local, bool 
 // group of loads (492 against 530 us).
 template <int SOLVER, bool ONE>
 __global__ void __launch_bounds__(kBX, 3) k_pred_flux_f32(BatchArgs ba, int kind) {
+    step_enter<ONE>();
     int local;
     const BoxRec rp = resolve<ONE>(ba, kind, local);
     if (!rp.active) return;
@@ -838,6 +861,7 @@ __device__ __forceinline__ void ld_prim(const float* __restrict__ S, int n, int 
 // per thread, whose larger window would not fit two.
 template <int SCHEME, int D, bool ONE>
 __global__ void __launch_bounds__(kBX, (scheme_recon(SCHEME) & 1) ? 6 : 3) k_sweep_f32(BatchArgs ba) {
+    step_enter<ONE>();
     int local;
     const BoxRec rp = resolve<ONE>(ba, scheme_kind(SCHEME, D == 1 ? kSubMarchY : kSubMarchZ), local);
     if (!rp.active) return;
@@ -977,6 +1001,7 @@ __device__ __forceinline__ void row_face(const V* sw, const V* sd, int ws, int d
 // y, y+1 side by side.  13 * nx * sizeof(V) bytes of shared memory.
 template <int SCHEME, class V, bool ONE>
 __global__ void __launch_bounds__(128, lanes_of<V>::n == 2 ? (scheme_solver(SCHEME) % 3 == 1 ? 4 : 5) : 8) k_xrow_f32(BatchArgs ba) {
+    step_enter<ONE>();
     constexpr int RECON = scheme_recon(SCHEME), W = lanes_of<V>::n;
     constexpr bool PPM = (RECON & 1) != 0;
     extern __shared__ __align__(16) unsigned char xrow_smem[];
@@ -1034,6 +1059,7 @@ __global__ void __launch_bounds__(128, lanes_of<V>::n == 2 ? (scheme_solver(SCHE
 // the whole-row kernel.
 template <int SCHEME, int TX, bool ONE>
 __global__ void __launch_bounds__(TX) k_xtile_f32(BatchArgs ba) {
+    step_enter<ONE>();
     constexpr int RECON = scheme_recon(SCHEME);
     constexpr bool PPM = (RECON & 1) != 0;
     constexpr int H = PPM ? 2 : 1;           // cells staged left of the tile
@@ -1150,6 +1176,7 @@ __device__ __forceinline__ CellEV<T> cell_ev(const T* __restrict__ S, int n, int
 template <class T, bool ONE, bool PROT = false, bool SHORT = false>
 __global__ void __launch_bounds__(kBX, 1) k_corner_emf(BatchArgs ba,
                                                                                        int half_step_state) {
+    step_enter<ONE>();
     int local;
     const BoxRec rp = resolve<ONE>(ba, kKindCellZ, local);
     if (!rp.active || (PROT && !rp.protect)) return;
@@ -1422,6 +1449,7 @@ __device__ __forceinline__ void do_corner_emf_f32(const BoxRec& rp, int local, i
 }
 template <bool ONE, bool PROT>
 __global__ void __launch_bounds__(kBX, 4) k_corner_emf_f32(BatchArgs ba, int half_step_state) {
+    step_enter<ONE>();
     int local;
     const BoxRec rp = resolve<ONE>(ba, kKindPairZ, local);
     if (!rp.active || (PROT && !rp.protect)) return;
@@ -1498,6 +1526,7 @@ __device__ __forceinline__ bool update_by_tma(const BoxRec& r) {
 // other instantiation has no per-plane test on the hot path.
 template <class T, bool ONE, bool ZR, bool SHORT = false>
 __global__ void __launch_bounds__(kBX, 1) k_update(BatchArgs ba, double dt_scale, int final_stage) {
+    step_enter<ONE>();
     int local;
     const BoxRec rp = resolve<ONE>(ba, kKindCellZ, local);
     Scalars* sc = rp.sc;
@@ -1510,7 +1539,7 @@ __global__ void __launch_bounds__(kBX, 1) k_update(BatchArgs ba, double dt_scale
     const T* __restrict__ E = (const T*)rp.E;
     const double dx = rp.dx;
     const T asqr = (T)(rp.cs * rp.cs);
-    const int do_cfl = final_stage && !sc->drive;
+    const int do_cfl = final_stage && !step_drive<ONE>(rp);
     const bool write_vt = final_stage && rp.npass > 0;
     unsigned long long* cmax_slots = sc->cmax_slots;
     unsigned long long* floor_hits = &sc->floor_hits;
@@ -1521,7 +1550,7 @@ __global__ void __launch_bounds__(kBX, 1) k_update(BatchArgs ba, double dt_scale
     double cmax = 0.0;
     if (valid) {
         const int n = dm.n;
-        const T dtdx = (T)(dt_scale * sc->dt / dx);
+        const T dtdx = (T)(dt_scale * step_dt<ONE>(rp) / dx);
         const int plane = dm.nx * dm.ny;
         const int im = wrap_dn(i, dm.nx), jm = wrap_dn(j, dm.ny);
         const int r0 = i + dm.nx * j, rxm = im + dm.nx * j, rym = i + dm.nx * jm, rxmym = im + dm.nx * jm;
@@ -1616,15 +1645,17 @@ template <class V>
 __device__ __forceinline__ V vt_pair(V rho0, V m0, V ir1, V m1) {
     return same<V>(0.5f) * fma(m0, vrcp(rho0), m1 * ir1);
 }
-// cell_max_speed of a pair, with its operations
+// cell_max_speed of a pair, with the roundings of its FP32 form (which of the
+// products are fused), so that dt is the one the single-cell kernels gave.
 __device__ __forceinline__ F2 cell_speed_fast(F2 rho, const F2* m, F2 bxc, F2 byc, F2 bzc, float asqr) {
-    const F2 is = each([](float r) { return 1.0f / sqrtf(r); }, rho), a2 = same<F2>(asqr);
-    const F2 bx = bxc * is, by = byc * is, bz = bzc * is, half = same<F2>(0.5f);
-    auto fast = [&](F2 bt, F2 n) {
-        const F2 b = fma(n, n, bt), d = a2 - b;
-        return vsqrt(half * ((a2 + b) + vsqrt(fma(d, d, same<F2>(4.0f * asqr) * bt))));
+    const F2 is = each([](float r) { return 1.0f / sqrtf(r); }, rho), a2 = same<F2>(asqr), half = same<F2>(0.5f);
+    const F2 bx = bxc * is, by = byc * is, bz = bzc * is, y2 = by * by, z2 = bz * bz;
+    auto fast = [&](F2 bt, F2 b) {
+        const F2 d = a2 - b;
+        return vsqrt(half * ((a2 + b) + vsqrt(fma(same<F2>(4.0f * asqr), bt, d * d))));
     };
-    const F2 cx = fast(fma(by, by, bz * bz), bx), cy = fast(fma(bx, bx, bz * bz), by), cz = fast(fma(bx, bx, by * by), bz);
+    const F2 tx = y2 + z2, ty = fma(bx, bx, z2), tz = fma(bx, bx, y2);
+    const F2 cx = fast(tx, fma(bx, bx, tx)), cy = fast(ty, y2 + ty), cz = fast(tz, fma(bz, bz, tz));
     auto quot = [](float a, float b) { return a / b; };
     return vmax2(vmax2(vabs(each(quot, m[0], rho)) + cx, vabs(each(quot, m[1], rho)) + cy), vabs(each(quot, m[2], rho)) + cz);
 }
@@ -1637,14 +1668,14 @@ __device__ __forceinline__ void do_update_f32(const BoxRec& rp, int local, doubl
     const float* __restrict__ F = (const float*)rp.F;
     const float* __restrict__ E = (const float*)rp.E;
     const float asqr = (float)(rp.cs * rp.cs);
-    const int do_cfl = final_stage && !sc->drive;
+    const int do_cfl = final_stage && !step_drive<ONE>(rp);
     const bool write_vt = final_stage && rp.npass > 0;
     int p, j, k0, k1;
     decode_cellz<ONE, true>(local, Dims{pairs_of(dm.nx), dm.ny, dm.nz, 0}, rp.ptws, rp.segzs, p, j, k0, k1);
     double cmax = 0.0;
     if (2 * p < dm.nx && j < dm.ny) {
         const int n = dm.n, plane = dm.nx * dm.ny;
-        const F2 ndt = same<F2>((float)(-dt_scale * sc->dt / rp.dx)), half = same<F2>(0.5f);
+        const F2 ndt = same<F2>((float)(-dt_scale * step_dt<ONE>(rp) / rp.dx)), half = same<F2>(0.5f);
         const int x0 = 2 * p, x1 = wrap_up(x0, dm.nx), xm = wrap_dn(x0, dm.nx), row = dm.nx * j, rowm = dm.nx * wrap_dn(j, dm.ny);
         const bool two = x0 + 1 < dm.nx;
         const int r0 = row + x0, r1 = row + x1, rm = row + xm, q0 = rowm + x0, q1 = rowm + x1, qm = rowm + xm;
@@ -1745,6 +1776,7 @@ __device__ __forceinline__ void do_update_f32(const BoxRec& rp, int local, doubl
 }
 template <bool ONE, bool ZR>
 __global__ void __launch_bounds__(kBX, 4) k_update_f32(BatchArgs ba, double dt_scale, int final_stage) {
+    step_enter<ONE>();
     int local;
     const BoxRec rp = resolve<ONE>(ba, kKindPairZ, local);
     if (!rp.active) return;
@@ -1818,6 +1850,7 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned by
 template <class T, bool ZR, bool ONE, int TW>
 __global__ void __launch_bounds__(kTmaTile, 1)
     k_update_tma(BatchArgs ba, double dt_scale, int final_stage) {
+    step_enter<ONE>();
     extern __shared__ __align__(128) unsigned char tma_smem[];
     __shared__ __align__(8) unsigned long long bars[2];
     constexpr int RB = kTmaTile / TW;    // rows per block
@@ -1831,7 +1864,7 @@ __global__ void __launch_bounds__(kTmaTile, 1)
     const T* __restrict__ F = (const T*)rp.F;
     const T* __restrict__ E = (const T*)rp.E;
     const T asqr = (T)(rp.cs * rp.cs);
-    const int do_cfl = final_stage && !sc->drive;
+    const int do_cfl = final_stage && !step_drive<ONE>(rp);
     const bool write_vt = final_stage && rp.npass > 0;
     const int t = (int)threadIdx.x;
     const int lx = t % TW, ly = t / TW;
@@ -1851,7 +1884,7 @@ __global__ void __launch_bounds__(kTmaTile, 1)
     const int k0 = seg * len, k1 = min(k0 + len, dm.nz);
     const int n = dm.n, plane = dm.nx * dm.ny;
     const int jm = wrap_dn(j, dm.ny);
-    const T dtdx = (T)(dt_scale * sc->dt / rp.dx);
+    const T dtdx = (T)(dt_scale * step_dt<ONE>(rp) / rp.dx);
     constexpr int HE = 16 / (int)sizeof(T);          // elements of a 16-byte segment
     const int ih = (i0 == 0 ? dm.nx : i0) - HE;       // segment ending at the cell left of the tile
     if (t == 0) {
@@ -2024,6 +2057,7 @@ __device__ __forceinline__ bool prot_corner(const unsigned char* __restrict__ ba
 // cells, then final_check_unphysical (:3243-3262) for them.
 template <class T, bool ONE>
 __global__ void __launch_bounds__(kBX) k_prot_hydro(BatchArgs ba, double dt_scale, int stage) {
+    step_enter<ONE>();
     int local;
     const BoxRec rp = prot_box<ONE>(ba, local);
     if (!rp.active || !rp.protect) return;
@@ -2038,7 +2072,7 @@ __global__ void __launch_bounds__(kBX) k_prot_hydro(BatchArgs ba, double dt_scal
     T* __restrict__ Sout = (T*)rp.S[1];
     const T* __restrict__ F = (const T*)rp.F;
     const T* __restrict__ Fp = (const T*)rp.Fp;
-    const T dtdx = (T)(dt_scale * sc->dt / rp.dx);
+    const T dtdx = (T)(dt_scale * step_dt<ONE>(rp) / rp.dx);
     for (long w = (long)local * blockDim.x + threadIdx.x; w < 7L * nb; w += (long)kProtBlocks * blockDim.x) {
         const int b = list[w / 7];
         const int slot = (int)(w % 7);
@@ -2096,6 +2130,7 @@ __global__ void __launch_bounds__(kBX) k_prot_hydro(BatchArgs ba, double dt_scal
 // they replace the corners (update_CT_3d, :2211-2245).
 template <class T, bool ONE>
 __global__ void __launch_bounds__(kBX) k_prot_faces(BatchArgs ba, double dt_scale, int stage) {
+    step_enter<ONE>();
     int local;
     const BoxRec rp = prot_box<ONE>(ba, local);
     if (!rp.active || !rp.protect) return;
@@ -2110,7 +2145,7 @@ __global__ void __launch_bounds__(kBX) k_prot_faces(BatchArgs ba, double dt_scal
     T* __restrict__ Sout = (T*)rp.S[1];
     const T* __restrict__ E = (const T*)rp.E;
     const T* __restrict__ Ep = (const T*)rp.Ep;
-    const T dtdx = (T)(dt_scale * sc->dt / rp.dx);
+    const T dtdx = (T)(dt_scale * step_dt<ONE>(rp) / rp.dx);
     // corner EMF of component m at cell (i,j,k): the protection value where replaced
     auto corner = [&](int m, int i, int j, int k) -> T {
         const int q = cell_at(dm, i, j, k);
@@ -2139,6 +2174,7 @@ __global__ void __launch_bounds__(kBX) k_prot_faces(BatchArgs ba, double dt_scal
 // Cell-centred field of the cells next to those faces (update_CT_3d, :2248-2259).
 template <class T, bool ONE>
 __global__ void __launch_bounds__(kBX) k_prot_centres(BatchArgs ba, int stage) {
+    step_enter<ONE>();
     int local;
     const BoxRec rp = prot_box<ONE>(ba, local);
     if (!rp.active || !rp.protect) return;
@@ -2167,11 +2203,12 @@ __global__ void __launch_bounds__(kBX) k_prot_centres(BatchArgs ba, int stage) {
 // the stage had bad cells (k_finalize then takes it instead of the update's).
 template <class T, bool ONE>
 __global__ void __launch_bounds__(kRedThreads) k_prot_cfl(BatchArgs ba) {
+    step_enter<ONE>();
     int local;
     const BoxRec rp = resolve<ONE>(ba, kKindRed, local);
     if (!rp.active || !rp.protect) return;
     Scalars* sc = rp.sc;
-    if (sc->nbad[1] == 0 || sc->drive) return;
+    if (sc->nbad[1] == 0 || step_drive<ONE>(rp)) return;
     const T* __restrict__ S = (const T*)rp.S[1];
     const T asqr = (T)(rp.cs * rp.cs);
     const int n = rp.n, plane = rp.nx * rp.ny;
@@ -2188,6 +2225,7 @@ __global__ void __launch_bounds__(kRedThreads) k_prot_cfl(BatchArgs ba) {
 // Clear the bad flags of a stage's list (the counts are reset by k_finalize).
 template <bool ONE>
 __global__ void __launch_bounds__(kBX) k_prot_clear(BatchArgs ba, int stage) {
+    step_enter<ONE>();
     int local;
     const BoxRec rp = prot_box<ONE>(ba, local);
     if (!rp.active || !rp.protect) return;
@@ -2219,6 +2257,7 @@ __device__ __forceinline__ T vel_of(const T* __restrict__ S, int n, int c, int c
 // cell: the same operands).  FP64; FP32 runs k_passive_pred_f32.
 template <class T, bool ONE, int NP, bool SHORT = false>
 __global__ void __launch_bounds__(kBX, 1) k_passive_pred(BatchArgs ba) {
+    step_enter<ONE>();
     int local;
     const BoxRec rp = resolve<ONE>(ba, kKindCellZ, local);
     const Scalars* sc = rp.sc;
@@ -2233,7 +2272,7 @@ __global__ void __launch_bounds__(kBX, 1) k_passive_pred(BatchArgs ba) {
     if (i >= dm.nx || j >= dm.ny) return;
     const int n = dm.n;
     const int plane = dm.nx * dm.ny;
-    const T dtdx = (T)(0.5 * sc->dt / dx);
+    const T dtdx = (T)(0.5 * step_dt<ONE>(rp) / dx);
     const int r0 = i + dm.nx * j;
     const int rxm = wrap_dn(i, dm.nx) + dm.nx * j, rxp = wrap_up(i, dm.nx) + dm.nx * j;
     const int rym = i + dm.nx * wrap_dn(j, dm.ny), ryp = i + dm.nx * wrap_up(j, dm.ny);
@@ -2307,6 +2346,7 @@ __device__ __forceinline__ T vtavg(const T* __restrict__ S0, const T* __restrict
 // FP64; FP32 runs k_passive_corr_f32.
 template <class T, bool ONE, int NP, bool SHORT = false>
 __global__ void __launch_bounds__(kBX, 1) k_passive_corr(BatchArgs ba) {
+    step_enter<ONE>();
     int local;
     const BoxRec rp = resolve<ONE>(ba, kKindCellZ, local);
     const Scalars* sc = rp.sc;
@@ -2318,7 +2358,7 @@ __global__ void __launch_bounds__(kBX, 1) k_passive_corr(BatchArgs ba) {
     const T* __restrict__ SH = (const T*)rp.SH;
     const T* __restrict__ VT = vt_field<T>(rp, 0);   // fields 0, 1 at +0, +n; field 2 at +6n (vt_field)
     const double dx = rp.dx;
-    const int drive = sc->drive;
+    const int drive = step_drive<ONE>(rp);
     const T* __restrict__ mbnd = (const T*)rp.mbnd;
     const int plane_stride = rp.plane_stride;
     int i, j, k0, k1;
@@ -2326,7 +2366,7 @@ __global__ void __launch_bounds__(kBX, 1) k_passive_corr(BatchArgs ba) {
     if (i >= dm.nx || j >= dm.ny) return;
     const int n = dm.n;
     const int plane = dm.nx * dm.ny;
-    const T dtdx = (T)(sc->dt / dx);
+    const T dtdx = (T)(step_dt<ONE>(rp) / dx);
     const int r0 = i + dm.nx * j;
     const int rxm = wrap_dn(i, dm.nx) + dm.nx * j, rxp = wrap_up(i, dm.nx) + dm.nx * j;
     const int rxm2 = wrap_any(i - 2, dm.nx) + dm.nx * j, rxp2 = wrap_any(i + 2, dm.nx) + dm.nx * j;
@@ -2439,7 +2479,7 @@ __device__ __forceinline__ void do_passive_pred_f32(const BoxRec& rp, int local)
     decode_cellz<ONE, true>(local, Dims{pairs_of(dm.nx), dm.ny, dm.nz, 0}, rp.ptws, rp.segzs, p, j, k0, k1);
     if (2 * p >= dm.nx || j >= dm.ny) return;
     const int n = dm.n, plane = dm.nx * dm.ny;
-    const F2 ndt = same<F2>((float)(-0.5 * sc->dt / rp.dx)), half = same<F2>(0.5f);
+    const F2 ndt = same<F2>((float)(-0.5 * step_dt<ONE>(rp) / rp.dx)), half = same<F2>(0.5f);
     const int x0 = 2 * p, x1 = wrap_up(x0, dm.nx), x2 = wrap_up(x1, dm.nx), xm = wrap_dn(x0, dm.nx);
     const bool two = x0 + 1 < dm.nx;
     const int row = dm.nx * j, rowm = dm.nx * wrap_dn(j, dm.ny), rowp = dm.nx * wrap_up(j, dm.ny);
@@ -2512,6 +2552,7 @@ __device__ __forceinline__ void do_passive_pred_f32(const BoxRec& rp, int local)
 }
 template <bool ONE, int NP>
 __global__ void __launch_bounds__(kBX, NP <= 2 ? 8 : NP <= 4 ? 6 : 3) k_passive_pred_f32(BatchArgs ba) {
+    step_enter<ONE>();
     int local;
     const BoxRec rp = resolve<ONE>(ba, kKindPairZ, local);
     if (!rp.active || rp.npass == 0) return;
@@ -2528,13 +2569,13 @@ __device__ __forceinline__ void do_passive_corr_f32(const BoxRec& rp, int local)
     float* __restrict__ S1 = (float*)rp.S[1];
     const float* __restrict__ SH = (const float*)rp.SH;
     const float* __restrict__ VT = vt_field<float>(rp, 0);   // fields 0, 1 at +0, +n; field 2 at +6n (vt_field)
-    const int drive = sc->drive, plane_stride = rp.plane_stride;
+    const int drive = step_drive<ONE>(rp), plane_stride = rp.plane_stride;
     const float* __restrict__ mbnd = (const float*)rp.mbnd;
     int p, j, k0, k1;
     decode_cellz<ONE, true>(local, Dims{pairs_of(dm.nx), dm.ny, dm.nz, 0}, rp.ptws, rp.segzs, p, j, k0, k1);
     if (2 * p >= dm.nx || j >= dm.ny) return;
     const int n = dm.n, plane = dm.nx * dm.ny;
-    const F2 ndt = same<F2>((float)(-sc->dt / rp.dx)), half = same<F2>(0.5f);
+    const F2 ndt = same<F2>((float)(-step_dt<ONE>(rp) / rp.dx)), half = same<F2>(0.5f);
     const int x0 = 2 * p, x1 = wrap_up(x0, dm.nx), x2 = wrap_up(x1, dm.nx), x3 = wrap_up(x2, dm.nx);
     const int xm = wrap_dn(x0, dm.nx), xm2 = wrap_dn(xm, dm.nx);
     const bool two = x0 + 1 < dm.nx;
@@ -2651,6 +2692,7 @@ __device__ __forceinline__ void do_passive_corr_f32(const BoxRec& rp, int local)
 }
 template <bool ONE, int NP>
 __global__ void __launch_bounds__(kBX, NP <= 2 ? 5 : NP <= 4 ? 3 : 2) k_passive_corr_f32(BatchArgs ba) {
+    step_enter<ONE>();
     int local;
     const BoxRec rp = resolve<ONE>(ba, kKindPairZ, local);
     if (!rp.active || rp.npass == 0) return;
@@ -2686,6 +2728,7 @@ __host__ __device__ __forceinline__ bool passive_by_tma(int nx) { return nx % kT
 
 template <class T, int NP>
 __global__ void __launch_bounds__(kTmaTile, 8) k_passive_corr_tma(BatchArgs ba) {
+    step_enter<true>();
     extern __shared__ __align__(128) unsigned char ptma_smem[];
     __shared__ __align__(8) unsigned long long bars[2];
     const BoxRec rp = ba.one;
@@ -2697,7 +2740,7 @@ __global__ void __launch_bounds__(kTmaTile, 8) k_passive_corr_tma(BatchArgs ba) 
     T* __restrict__ S1 = (T*)rp.S[1];
     const T* __restrict__ SH = (const T*)rp.SH;
     const T* __restrict__ VT = vt_field<T>(rp, 0);   // v_x, v_y at +0, +n; v_z at +6n
-    const int drive = sc->drive;
+    const int drive = step_drive<true>(rp);
     const T* __restrict__ mbnd = (const T*)rp.mbnd;
     const int plane_stride = rp.plane_stride;
     constexpr int HE = 16 / (int)sizeof(T);
@@ -2707,7 +2750,7 @@ __global__ void __launch_bounds__(kTmaTile, 8) k_passive_corr_tma(BatchArgs ba) 
     const int i = i0 + t;
     const int k0 = seg << rp.segzs, k1 = min(k0 + (1 << rp.segzs), dm.nz);
     const int n = dm.n, plane = dm.nx * dm.ny;
-    const T dtdx = (T)(sc->dt / rp.dx);
+    const T dtdx = (T)(step_dt<true>(rp) / rp.dx);
     const int nrows = 7 * npass + 5;
     const int ih = (i0 == 0 ? dm.nx : i0) - HE;       // left halo: cells i0-HE .. i0-1
     const int ir = (i0 + kTmaTile) % dm.nx;            // right halo: cells i0+128 .. i0+128+HE-1
@@ -2885,6 +2928,7 @@ constexpr size_t passive_pred_tma_smem_bytes() { return 2 * ppred_stage_bytes<T,
 template <class T, int NP>
 __global__ void __launch_bounds__(kTmaTile, 1)
     k_passive_pred_tma(BatchArgs ba) {
+    step_enter<true>();
     extern __shared__ __align__(128) unsigned char pptma_smem[];
     __shared__ __align__(8) unsigned long long bars[2];
     __shared__ const T* row_src[ppred_rows<NP>()];
@@ -2947,7 +2991,7 @@ __global__ void __launch_bounds__(kTmaTile, 1)
         }
     };
     if (t < 32) issue(0, k0);
-    const T dtdx = (T)(0.5 * sc->dt / rp.dx);
+    const T dtdx = (T)(0.5 * step_dt<true>(rp) / rp.dx);
     const int r0 = i + dm.nx * j;
     // carried from plane k-1: scalar, velocities, x and y flux differences, z face below
     T ps[NP], pdx[NP], pdy[NP], pfz[NP];
@@ -3023,10 +3067,11 @@ __global__ void __launch_bounds__(kTmaTile, 1)
 // of a drive step, unless the host has set all ranks' sums (ext_sums).
 template <class T, bool ONE>
 __global__ void __launch_bounds__(kRedThreads) k_force_sums(BatchArgs ba, int sums_only) {
+    step_enter<ONE>();
     int local;
     const BoxRec rp = resolve<ONE>(ba, kKindRed, local);
     const Scalars* sc = rp.sc;
-    if (!rp.active || (!sums_only && (!sc->drive || sc->ext_sums))) return;
+    if (!rp.active || (!sums_only && (!step_drive<ONE>(rp) || sc->ext_sums))) return;
     const T* __restrict__ S0 = (const T*)rp.S[0];
     const T* __restrict__ delv = (const T*)rp.delv;
     double* __restrict__ partials = rp.partials;
@@ -3083,9 +3128,10 @@ __device__ __forceinline__ void force_normalise(Scalars* sc, const double* s, do
 // or all ranks' when the host set them (ext_sums, consumed here);
 // sums_only stops after storing this box's sums.
 static __global__ void k_force_reduce(BatchArgs ba, int sums_only) {
+    step_enter<true>();
     const BoxRec rp = box_at(ba, blockIdx.x);   // one block of 32 threads per box
     Scalars* sc = rp.sc;
-    if (!rp.active || (!sums_only && !sc->drive)) return;
+    if (!rp.active || (!sums_only && !(ba.use_one ? rp.drive : sc->drive))) return;
     if (!sums_only && sc->ext_sums) {
         if (threadIdx.x == 0) {
             sc->ext_sums = 0u;
@@ -3124,10 +3170,11 @@ static __global__ void k_force_reduce(BatchArgs ba, int sums_only) {
 // state, and the unforced boundary-plane momentum for k_passive_corr.
 template <class T, bool ONE>
 __global__ void __launch_bounds__(kBX) k_force_kick(BatchArgs ba) {
+    step_enter<ONE>();
     int local;
     const BoxRec rp = resolve<ONE>(ba, kKindCell, local);
     Scalars* sc = rp.sc;
-    if (!rp.active || !sc->drive) return;
+    if (!rp.active || !step_drive<ONE>(rp)) return;
     const Dims dm = dims_of(rp);
     const T* __restrict__ S0 = (const T*)rp.S[0];
     T* __restrict__ S1 = (T*)rp.S[1];
@@ -3189,12 +3236,13 @@ __global__ void __launch_bounds__(kBX) k_force_kick(BatchArgs ba) {
 // lane 0 does the rest (a single thread's serial loads and stores took 13-20
 // us of every step, between events; the warp takes 6-8 us).
 static __global__ void __launch_bounds__(32) k_finalize(BatchArgs ba, int device_driven) {
+    step_enter<true>();
     const int b = (int)blockIdx.x;
     const BoxRec rp = box_at(ba, b);
     Scalars* sc = rp.sc;
     if (!rp.active) return;
     const double cour = rp.cour, dx = rp.dx;
-    const int drive = sc->drive;
+    const int drive = ba.use_one ? rp.drive : sc->drive;
     double cell = 0.0, smax = 0.0, dvm = 0.0;
     // after a protected final update with bad cells the CFL maximum of the
     // corrected state is in cfl_slots (k_prot_cfl)
@@ -3222,6 +3270,17 @@ static __global__ void __launch_bounds__(32) k_finalize(BatchArgs ba, int device
     sc->dvmax_last = dvm;
     sc->dt_next = c * dx / cmax;
     sc->cur ^= 1;   // the new state is now current
+    if (ba.use_one) {
+        // what the host waits for, where it can read it
+        unsigned st = sc->status;
+        sc->report[0] = sc->dt_next;
+        sc->report[1] = __longlong_as_double((long long)st);
+        if (ba.report) {
+            ba.report[0] = sc->report[0];
+            ba.report[1] = sc->report[1];
+            __threadfence_system();
+        }
+    }
     if (!ba.use_one) {
         BoxRec& tr = ba.boxes[b];
         void* s0 = tr.S[0];
@@ -3245,6 +3304,7 @@ static __global__ void __launch_bounds__(32) k_finalize(BatchArgs ba, int device
 // Drive decision of a device-driven step (driver.f90:57-70): a box drives
 // when t_turb falls in (t, t + dt]; then t_turb advances and dt halves.
 static __global__ void k_batch_begin(BatchArgs ba) {
+    step_enter<true>();
     int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= ba.nbox) return;
     const BoxRec rp = box_at(ba, b);
@@ -3263,6 +3323,7 @@ static __global__ void k_batch_begin(BatchArgs ba) {
 // t, steps made, running flag, current buffer, status bits, next dt.
 constexpr int kClockWords = 6;
 static __global__ void k_clocks(BatchArgs ba, double* __restrict__ out) {
+    step_enter<true>();
     int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= ba.nbox) return;
     const Scalars* sc = box_at(ba, b).sc;
@@ -3278,6 +3339,7 @@ static __global__ void k_clocks(BatchArgs ba, double* __restrict__ out) {
 // cell fast-speed maximum of a state (imhd_max_speed)
 template <class T, bool ONE>
 __global__ void __launch_bounds__(kBX) k_cfl(BatchArgs ba) {
+    step_enter<ONE>();
     int local;
     const BoxRec rp = resolve<ONE>(ba, kKindCell, local);
     Scalars* sc = rp.sc;
@@ -3302,6 +3364,7 @@ __global__ void __launch_bounds__(kBX) k_cfl(BatchArgs ba) {
 // per-block partials; reduced by k_diag_reduce in block order.
 template <class T, bool ONE>
 __global__ void __launch_bounds__(kRedThreads) k_diag(BatchArgs ba) {
+    step_enter<ONE>();
     int local;
     const BoxRec rp = resolve<ONE>(ba, kKindRed, local);
     const Dims dm = dims_of(rp);
@@ -3340,6 +3403,7 @@ __global__ void __launch_bounds__(kRedThreads) k_diag(BatchArgs ba) {
 }
 
 static __global__ void k_diag_reduce(BatchArgs ba) {
+    step_enter<true>();
     if (threadIdx.x != 0) return;
     const BoxRec rp = box_at(ba, blockIdx.x);   // one block per box
     Scalars* sc = rp.sc;

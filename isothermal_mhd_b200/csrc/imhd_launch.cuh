@@ -6,9 +6,10 @@
 // Every launch covers all boxes of the table: the grid is the sum of the
 // boxes' blocks for that kernel's decomposition (BatchDev::totals).  A single
 // box travels in the kernel parameters (kernels instantiated with ONE); in a
-// batch each block reads its box from the block -> box table.  A step never
-// reads the host: dt, the drive flag and the current state buffer are device
-// scalars of each box, so the sequence can be captured in a CUDA graph.
+// batch each block reads its box from the block -> box table.  A table's step
+// never reads the host: dt, the drive flag and the current state buffer are
+// device scalars of each box, so the sequence can be captured in a CUDA graph.
+// A single box's dt and drive flag travel in the launch parameters.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -35,7 +36,33 @@ inline int ceil_shift(int n, int log) { return (n + (1 << log) - 1) >> log; }
 inline void mark(BatchDev& b, int stage) {
     if (!b.prof) return;
     cudaEventRecord(b.ev[stage], b.st);
+    b.chain = false;
     b.prof_mask |= 1u << stage;
+}
+
+// Launch a kernel of a step.  A single box's kernels after the first may be
+// scheduled while the one before still runs (programmatic stream
+// serialization): their blocks take the SM slots that its last wave leaves
+// free and wait there (step_enter), so that a small box does not pay a launch
+// and a drain between any two of its kernels (32^3: 74 -> 50 us a step, 96^3 213
+// -> 190, 128^3 with a kick 494 -> 455).  Boxes above kChainCells gain nothing
+// (256^3: 3.04, 3.03 ms) or lose: an SM that is never idle keeps the shared
+// memory split of the kernel before, and 512^3 went from 23.6 to 26.4 ms.
+constexpr int kChainCells = 1 << 22;
+template <class... P, class... A>
+static void launch(BatchDev& b, void (*kernel)(P...), dim3 grid, int threads, size_t smem, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = b.st;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = b.a.use_one && b.chain ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+    b.chain = b.a.use_one && b.a.one.n <= kChainCells;
 }
 
 // Grid of a launch of decomposition `kind`: the table's total block count, or
@@ -82,15 +109,15 @@ template <class T, bool ONE, bool PROT>
 static void launch_emf(BatchDev& b, dim3 gz, int half_step_state) {
     b.launches += 1;
     if constexpr (sizeof(T) == 4) {
-        k_corner_emf_f32<ONE, PROT><<<gz, kBX, 0, b.st>>>(b.a, half_step_state);
+        launch(b, k_corner_emf_f32<ONE, PROT>, gz, kBX, 0, b.a, half_step_state);
     } else {
         if constexpr (ONE) {
             if (short_columns<ONE>(b)) {
-                k_corner_emf<T, ONE, PROT, true><<<gz, kBX, 0, b.st>>>(b.a, half_step_state);
+                launch(b, k_corner_emf<T, ONE, PROT, true>, gz, kBX, 0, b.a, half_step_state);
                 return;
             }
         }
-        k_corner_emf<T, ONE, PROT><<<gz, kBX, 0, b.st>>>(b.a, half_step_state);
+        launch(b, k_corner_emf<T, ONE, PROT>, gz, kBX, 0, b.a, half_step_state);
     }
 }
 
@@ -107,15 +134,15 @@ static void launch_fluxes_pred(BatchDev& b) {
     if (!b.has_scheme[SCHEME] || b.totals[kind] == 0) return;
     b.launches += 1;
     if constexpr (pair_scheme<T, SCHEME, ONE>()) {
-        k_pred_flux_f32<scheme_solver(SCHEME), ONE><<<grid_of<ONE>(b, kind, true), kBX, 0, b.st>>>(b.a, kind);
+        launch(b, k_pred_flux_f32<scheme_solver(SCHEME), ONE>, grid_of<ONE>(b, kind, true), kBX, 0, b.a, kind);
     } else {
         if constexpr (ONE) {
             if (short_columns<ONE>(b)) {
-                k_pred_flux<T, SCHEME, ONE, true><<<grid_of<ONE>(b, kind), kBX, 0, b.st>>>(b.a);
+                launch(b, k_pred_flux<T, SCHEME, ONE, true>, grid_of<ONE>(b, kind), kBX, 0, b.a);
                 return;
             }
         }
-        k_pred_flux<T, SCHEME, ONE><<<grid_of<ONE>(b, kind), kBX, 0, b.st>>>(b.a);
+        launch(b, k_pred_flux<T, SCHEME, ONE>, grid_of<ONE>(b, kind), kBX, 0, b.a);
     }
 }
 
@@ -164,8 +191,8 @@ static void ensure_update_tma_attr() {
 template <class T, bool ONE, int TW>
 static void launch_update_tma(BatchDev& b, dim3 g, double dt_scale, int final_stage) {
     const size_t smem = update_tma_smem_bytes<T, TW>();
-    if (b.any_zrange) k_update_tma<T, true, ONE, TW><<<g, kTmaTile, smem, b.st>>>(b.a, dt_scale, final_stage);
-    else k_update_tma<T, false, ONE, TW><<<g, kTmaTile, smem, b.st>>>(b.a, dt_scale, final_stage);
+    if (b.any_zrange) launch(b, k_update_tma<T, true, ONE, TW>, g, kTmaTile, smem, b.a, dt_scale, final_stage);
+    else launch(b, k_update_tma<T, false, ONE, TW>, g, kTmaTile, smem, b.a, dt_scale, final_stage);
     b.launches += 1;
 }
 
@@ -179,8 +206,8 @@ template <class T, bool ONE>
 static void launch_update(BatchDev& b, double dt_scale, int final_stage) {
     const dim3 gz = zgrid<T, ONE>(b);
     if constexpr (sizeof(T) == 4) {
-        if (b.any_zrange) k_update_f32<ONE, true><<<gz, kBX, 0, b.st>>>(b.a, dt_scale, final_stage);
-        else k_update_f32<ONE, false><<<gz, kBX, 0, b.st>>>(b.a, dt_scale, final_stage);
+        if (b.any_zrange) launch(b, k_update_f32<ONE, true>, gz, kBX, 0, b.a, dt_scale, final_stage);
+        else launch(b, k_update_f32<ONE, false>, gz, kBX, 0, b.a, dt_scale, final_stage);
         b.launches += 1;
     } else {
         // the bulk copies need 16-byte aligned sources: every row of a 128-cell
@@ -197,14 +224,14 @@ static void launch_update(BatchDev& b, double dt_scale, int final_stage) {
         }
         if constexpr (ONE) {
             if (short_columns<ONE>(b)) {
-                if (b.any_zrange) k_update<T, ONE, true, true><<<gz, kBX, 0, b.st>>>(b.a, dt_scale, final_stage);
-                else k_update<T, ONE, false, true><<<gz, kBX, 0, b.st>>>(b.a, dt_scale, final_stage);
+                if (b.any_zrange) launch(b, k_update<T, ONE, true, true>, gz, kBX, 0, b.a, dt_scale, final_stage);
+                else launch(b, k_update<T, ONE, false, true>, gz, kBX, 0, b.a, dt_scale, final_stage);
                 b.launches += 1;
                 return;
             }
         }
-        if (b.any_zrange) k_update<T, ONE, true><<<gz, kBX, 0, b.st>>>(b.a, dt_scale, final_stage);
-        else k_update<T, ONE, false><<<gz, kBX, 0, b.st>>>(b.a, dt_scale, final_stage);
+        if (b.any_zrange) launch(b, k_update<T, ONE, true>, gz, kBX, 0, b.a, dt_scale, final_stage);
+        else launch(b, k_update<T, ONE, false>, gz, kBX, 0, b.a, dt_scale, final_stage);
         b.launches += 1;
         if (!ONE && (b.totals[kKindUpdTma] > 0 || b.totals[kKindUpdTma64] > 0)) {
             ensure_update_tma_attr<T>();
@@ -264,36 +291,36 @@ template <class T, bool ONE>
 static void launch_passive_pred(BatchDev& b, dim3 gz) {
     const BoxRec& r = b.a.one;
     if constexpr (sizeof(T) == 4) {
-        if (b.npass_max <= 1) k_passive_pred_f32<ONE, 1><<<gz, kBX, 0, b.st>>>(b.a);
-        else if (b.npass_max <= 2) k_passive_pred_f32<ONE, 2><<<gz, kBX, 0, b.st>>>(b.a);
-        else if (b.npass_max <= 4) k_passive_pred_f32<ONE, 4><<<gz, kBX, 0, b.st>>>(b.a);
-        else k_passive_pred_f32<ONE, kMaxPass><<<gz, kBX, 0, b.st>>>(b.a);
+        if (b.npass_max <= 1) launch(b, k_passive_pred_f32<ONE, 1>, gz, kBX, 0, b.a);
+        else if (b.npass_max <= 2) launch(b, k_passive_pred_f32<ONE, 2>, gz, kBX, 0, b.a);
+        else if (b.npass_max <= 4) launch(b, k_passive_pred_f32<ONE, 4>, gz, kBX, 0, b.a);
+        else launch(b, k_passive_pred_f32<ONE, kMaxPass>, gz, kBX, 0, b.a);
         b.launches += 1;
     } else {
         if (ONE && ((uintptr_t)r.S[0] | (uintptr_t)r.SH) % 16 == 0 && passive_by_tma(r.nx)) {
             ensure_passive_pred_tma_attr<T>();
             const dim3 g((unsigned)(r.nx / kTmaTile), (unsigned)r.ny, (unsigned)ceil_shift(r.nz, r.segzs));
             if (b.npass_max <= 2)
-                k_passive_pred_tma<T, 2><<<g, kTmaTile, passive_pred_tma_smem_bytes<T, 2>(), b.st>>>(b.a);
+                launch(b, k_passive_pred_tma<T, 2>, g, kTmaTile, passive_pred_tma_smem_bytes<T, 2>(), b.a);
             else if (b.npass_max <= 4)
-                k_passive_pred_tma<T, 4><<<g, kTmaTile, passive_pred_tma_smem_bytes<T, 4>(), b.st>>>(b.a);
+                launch(b, k_passive_pred_tma<T, 4>, g, kTmaTile, passive_pred_tma_smem_bytes<T, 4>(), b.a);
             else
-                k_passive_pred_tma<T, kMaxPass><<<g, kTmaTile, passive_pred_tma_smem_bytes<T, kMaxPass>(), b.st>>>(b.a);
+                launch(b, k_passive_pred_tma<T, kMaxPass>, g, kTmaTile, passive_pred_tma_smem_bytes<T, kMaxPass>(), b.a);
             b.launches += 1;
             return;
         }
         if constexpr (ONE) {
             if (short_columns<ONE>(b)) {
-                if (b.npass_max <= 2) k_passive_pred<T, ONE, 2, true><<<gz, kBX, 0, b.st>>>(b.a);
-                else if (b.npass_max <= 4) k_passive_pred<T, ONE, 4, true><<<gz, kBX, 0, b.st>>>(b.a);
-                else k_passive_pred<T, ONE, kMaxPass, true><<<gz, kBX, 0, b.st>>>(b.a);
+                if (b.npass_max <= 2) launch(b, k_passive_pred<T, ONE, 2, true>, gz, kBX, 0, b.a);
+                else if (b.npass_max <= 4) launch(b, k_passive_pred<T, ONE, 4, true>, gz, kBX, 0, b.a);
+                else launch(b, k_passive_pred<T, ONE, kMaxPass, true>, gz, kBX, 0, b.a);
                 b.launches += 1;
                 return;
             }
         }
-        if (b.npass_max <= 2) k_passive_pred<T, ONE, 2><<<gz, kBX, 0, b.st>>>(b.a);
-        else if (b.npass_max <= 4) k_passive_pred<T, ONE, 4><<<gz, kBX, 0, b.st>>>(b.a);
-        else k_passive_pred<T, ONE, kMaxPass><<<gz, kBX, 0, b.st>>>(b.a);
+        if (b.npass_max <= 2) launch(b, k_passive_pred<T, ONE, 2>, gz, kBX, 0, b.a);
+        else if (b.npass_max <= 4) launch(b, k_passive_pred<T, ONE, 4>, gz, kBX, 0, b.a);
+        else launch(b, k_passive_pred<T, ONE, kMaxPass>, gz, kBX, 0, b.a);
         b.launches += 1;
     }
 }
@@ -302,36 +329,36 @@ template <class T, bool ONE>
 static void launch_passive_corr(BatchDev& b, dim3 gz) {
     const BoxRec& r = b.a.one;
     if constexpr (sizeof(T) == 4) {
-        if (b.npass_max <= 1) k_passive_corr_f32<ONE, 1><<<gz, kBX, 0, b.st>>>(b.a);
-        else if (b.npass_max <= 2) k_passive_corr_f32<ONE, 2><<<gz, kBX, 0, b.st>>>(b.a);
-        else if (b.npass_max <= 4) k_passive_corr_f32<ONE, 4><<<gz, kBX, 0, b.st>>>(b.a);
-        else k_passive_corr_f32<ONE, kMaxPass><<<gz, kBX, 0, b.st>>>(b.a);
+        if (b.npass_max <= 1) launch(b, k_passive_corr_f32<ONE, 1>, gz, kBX, 0, b.a);
+        else if (b.npass_max <= 2) launch(b, k_passive_corr_f32<ONE, 2>, gz, kBX, 0, b.a);
+        else if (b.npass_max <= 4) launch(b, k_passive_corr_f32<ONE, 4>, gz, kBX, 0, b.a);
+        else launch(b, k_passive_corr_f32<ONE, kMaxPass>, gz, kBX, 0, b.a);
         b.launches += 1;
     } else {
         if (ONE && ((uintptr_t)r.S[0] | (uintptr_t)r.SH | (uintptr_t)r.F) % 16 == 0 && passive_by_tma(r.nx)) {
             ensure_passive_tma_attr<T>();
             const dim3 g((unsigned)(r.nx / kTmaTile), (unsigned)r.ny, (unsigned)ceil_shift(r.nz, r.segzs));
             if (b.npass_max <= 2)
-                k_passive_corr_tma<T, 2><<<g, kTmaTile, passive_tma_smem_bytes<T, 2>(), b.st>>>(b.a);
+                launch(b, k_passive_corr_tma<T, 2>, g, kTmaTile, passive_tma_smem_bytes<T, 2>(), b.a);
             else if (b.npass_max <= 4)
-                k_passive_corr_tma<T, 4><<<g, kTmaTile, passive_tma_smem_bytes<T, 4>(), b.st>>>(b.a);
+                launch(b, k_passive_corr_tma<T, 4>, g, kTmaTile, passive_tma_smem_bytes<T, 4>(), b.a);
             else
-                k_passive_corr_tma<T, kMaxPass><<<g, kTmaTile, passive_tma_smem_bytes<T, kMaxPass>(), b.st>>>(b.a);
+                launch(b, k_passive_corr_tma<T, kMaxPass>, g, kTmaTile, passive_tma_smem_bytes<T, kMaxPass>(), b.a);
             b.launches += 1;
             return;
         }
         if constexpr (ONE) {
             if (short_columns<ONE>(b)) {
-                if (b.npass_max <= 2) k_passive_corr<T, ONE, 2, true><<<gz, kBX, 0, b.st>>>(b.a);
-                else if (b.npass_max <= 4) k_passive_corr<T, ONE, 4, true><<<gz, kBX, 0, b.st>>>(b.a);
-                else k_passive_corr<T, ONE, kMaxPass, true><<<gz, kBX, 0, b.st>>>(b.a);
+                if (b.npass_max <= 2) launch(b, k_passive_corr<T, ONE, 2, true>, gz, kBX, 0, b.a);
+                else if (b.npass_max <= 4) launch(b, k_passive_corr<T, ONE, 4, true>, gz, kBX, 0, b.a);
+                else launch(b, k_passive_corr<T, ONE, kMaxPass, true>, gz, kBX, 0, b.a);
                 b.launches += 1;
                 return;
             }
         }
-        if (b.npass_max <= 2) k_passive_corr<T, ONE, 2><<<gz, kBX, 0, b.st>>>(b.a);
-        else if (b.npass_max <= 4) k_passive_corr<T, ONE, 4><<<gz, kBX, 0, b.st>>>(b.a);
-        else k_passive_corr<T, ONE, kMaxPass><<<gz, kBX, 0, b.st>>>(b.a);
+        if (b.npass_max <= 2) launch(b, k_passive_corr<T, ONE, 2>, gz, kBX, 0, b.a);
+        else if (b.npass_max <= 4) launch(b, k_passive_corr<T, ONE, 4>, gz, kBX, 0, b.a);
+        else launch(b, k_passive_corr<T, ONE, kMaxPass>, gz, kBX, 0, b.a);
         b.launches += 1;
     }
 }
@@ -363,17 +390,17 @@ static void launch_fluxes_corr_x(BatchDev& b) {
         ensure_xrow_attr<T, SCHEME, ONE>();
         const int bd = b.row_nx_max >= 128 ? 128 : ((b.row_nx_max + 31) / 32) * 32;
         if constexpr (pair_sweep<T, SCHEME, ONE>()) {
-            if (pairs) xrow_kernel<T, SCHEME, ONE, true>()<<<gr, bd, smem, b.st>>>(b.a);
-            else xrow_kernel<T, SCHEME, ONE, false>()<<<gr, bd, smem, b.st>>>(b.a);
+            if (pairs) launch(b, xrow_kernel<T, SCHEME, ONE, true>(), gr, bd, smem, b.a);
+            else launch(b, xrow_kernel<T, SCHEME, ONE, false>(), gr, bd, smem, b.a);
         } else {
-            xrow_kernel<T, SCHEME, ONE, false>()<<<gr, bd, smem, b.st>>>(b.a);
+            launch(b, xrow_kernel<T, SCHEME, ONE, false>(), gr, bd, smem, b.a);
         }
         b.launches += 1;
     }
     if (b.totals[ktile]) {
         const dim3 gt = grid_of<ONE>(b, ktile);
-        if constexpr (pair_scheme<T, SCHEME, ONE>()) k_xtile_f32<SCHEME, kTX, ONE><<<gt, kTX, 0, b.st>>>(b.a);
-        else k_corr_flux_x<T, SCHEME, kTX, ONE><<<gt, kTX, 0, b.st>>>(b.a);
+        if constexpr (pair_scheme<T, SCHEME, ONE>()) launch(b, k_xtile_f32<SCHEME, kTX, ONE>, gt, kTX, 0, b.a);
+        else launch(b, k_corr_flux_x<T, SCHEME, kTX, ONE>, gt, kTX, 0, b.a);
         b.launches += 1;
     }
 }
@@ -383,8 +410,8 @@ static void launch_fluxes_corr_march(BatchDev& b) {
     const int kind = scheme_kind(SCHEME, D == 1 ? kSubMarchY : kSubMarchZ);
     if (!b.has_scheme[SCHEME] || b.totals[kind] == 0) return;
     const dim3 g = grid_of<ONE>(b, kind, pair_sweep<T, SCHEME, ONE>());
-    if constexpr (pair_scheme<T, SCHEME, ONE>()) k_sweep_f32<SCHEME, D, ONE><<<g, kBX, 0, b.st>>>(b.a);
-    else k_corr_flux_march<T, SCHEME, D, ONE><<<g, kBX, 0, b.st>>>(b.a);
+    if constexpr (pair_scheme<T, SCHEME, ONE>()) launch(b, k_sweep_f32<SCHEME, D, ONE>, g, kBX, 0, b.a);
+    else launch(b, k_corr_flux_march<T, SCHEME, D, ONE>, g, kBX, 0, b.a);
     b.launches += 1;
 }
 
@@ -396,15 +423,15 @@ static void launch_fluxes_corr_march(BatchDev& b) {
 template <class T, bool ONE>
 static void launch_protection(BatchDev& b, double dt_scale, int stage) {
     const unsigned g = ONE ? (unsigned)kProtBlocks : (unsigned)(kProtBlocks * b.a.nbox);
-    k_prot_hydro<T, ONE><<<g, kBX, 0, b.st>>>(b.a, dt_scale, stage);
-    k_prot_faces<T, ONE><<<g, kBX, 0, b.st>>>(b.a, dt_scale, stage);
-    k_prot_centres<T, ONE><<<g, kBX, 0, b.st>>>(b.a, stage);
+    launch(b, k_prot_hydro<T, ONE>, g, kBX, 0, b.a, dt_scale, stage);
+    launch(b, k_prot_faces<T, ONE>, g, kBX, 0, b.a, dt_scale, stage);
+    launch(b, k_prot_centres<T, ONE>, g, kBX, 0, b.a, stage);
     b.launches += 3;
     if (stage == 1) {
-        k_prot_cfl<T, ONE><<<b.totals[kKindRed], kRedThreads, 0, b.st>>>(b.a);
+        launch(b, k_prot_cfl<T, ONE>, b.totals[kKindRed], kRedThreads, 0, b.a);
         b.launches += 1;
     }
-    k_prot_clear<ONE><<<g, kBX, 0, b.st>>>(b.a, stage);
+    launch(b, k_prot_clear<ONE>, g, kBX, 0, b.a, stage);
     b.launches += 1;
 }
 
@@ -414,14 +441,15 @@ static cudaError_t run_step_t(BatchDev& b, int device_driven) {
     const dim3 gz = zgrid<T, ONE>(b);
     const int nfin = (b.a.nbox + 31) / 32;
     b.prof_mask = 0;
+    b.chain = false;   // the first kernel waits for whatever the stream holds
     if (device_driven) {
-        k_batch_begin<<<nfin, 32, 0, b.st>>>(b.a);
+        launch(b, k_batch_begin, nfin, 32, 0, b.a);
         b.launches += 1;
     }
     if (b.drive_mode) {
         mark(b, kStForceSums);
-        k_force_sums<T, ONE><<<b.totals[kKindRed], kRedThreads, 0, b.st>>>(b.a, 0);
-        k_force_reduce<<<b.a.nbox, 32, 0, b.st>>>(b.a, 0);
+        launch(b, k_force_sums<T, ONE>, b.totals[kKindRed], kRedThreads, 0, b.a, 0);
+        launch(b, k_force_reduce, b.a.nbox, 32, 0, b.a, 0);
         b.launches += 2;
     }
     // predictor: first-order fluxes, EMFs, half-dt update into the other buffer
@@ -449,7 +477,7 @@ static cudaError_t run_step_t(BatchDev& b, int device_driven) {
     if (b.any_protect) launch_protection<T, ONE>(b, 1.0, 1);
     if (b.drive_mode) {
         mark(b, kStForceKick);
-        k_force_kick<T, ONE><<<gc, kBX, 0, b.st>>>(b.a);
+        launch(b, k_force_kick<T, ONE>, gc, kBX, 0, b.a);
         b.launches += 1;
     }
     if (b.any_pass) {
@@ -459,7 +487,7 @@ static cudaError_t run_step_t(BatchDev& b, int device_driven) {
         launch_passive_corr<T, ONE>(b, gz);
     }
     mark(b, kStFinalize);
-    k_finalize<<<b.a.nbox, 32, 0, b.st>>>(b.a, device_driven);
+    launch(b, k_finalize, b.a.nbox, 32, 0, b.a, device_driven);
     b.launches += 1;
     if (b.prof) cudaEventRecord(b.ev[kStages], b.st);
     return cudaGetLastError();

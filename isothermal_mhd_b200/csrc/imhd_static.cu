@@ -128,31 +128,25 @@ extern "C" int imhd_step_static(int precision, int nx, int ny, int nz, int riema
     std::vector<imhd::BoxRec> recs(1, rec);
     std::vector<int> prefix;
     if (!imhd::build_prefix(recs, esz, prefix, b, true)) return fail(IMHD_E_ARG, "box too large for one launch");
-    b.a.boxes = (imhd::BoxRec*)table;
-    b.a.prefix = (const int*)(table + 256);
+    rec.dt = dt;
     b.a.use_one = 1;                                      // the box travels in the launch parameters
+    b.a.report = nullptr;
     b.a.one = rec;
     b.drive_mode = 0;
-    imhd::Scalars init;
-    std::memset(&init, 0, sizeof(init));
-    init.active = 1;                                      // cur = 0: state_in is current
-    init.dt = dt;
 
-    double host_io[2] = {dt, 0.0};
-    unsigned status = 0;
+    double report[2] = {0.0, 0.0};
     // the scalars (maxima slots included) start from zero on every call
-    e = cudaMemcpyAsync(rec.sc, &init, sizeof(init), cudaMemcpyHostToDevice, b.st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(table, &rec, sizeof(rec), cudaMemcpyHostToDevice, b.st);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(table + 256, prefix.data(), prefix.size() * sizeof(int), cudaMemcpyHostToDevice, b.st);
+    e = cudaMemsetAsync(rec.sc, 0, sizeof(imhd::Scalars), b.st);
     if (e == cudaSuccess) e = precision == 64 ? imhd::run_step<double>(b, 0) : imhd::run_step<float>(b, 0);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&host_io[1], &rec.sc->dt_next, sizeof(double), cudaMemcpyDeviceToHost, b.st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&status, &rec.sc->status, sizeof(unsigned), cudaMemcpyDeviceToHost, b.st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(report, rec.sc->report, sizeof(report), cudaMemcpyDeviceToHost, b.st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(b.st);
     if (e != cudaSuccess) return fail(IMHD_E_CUDA, std::string("imhd_step_static: ") + cudaGetErrorString(e));
+    long long bits;
+    std::memcpy(&bits, &report[1], sizeof(bits));
+    const unsigned status = (unsigned)bits;
     if (status & IMHD_S_WAIT) return fail(IMHD_E_CUDA, "a bounded wait for an asynchronous copy gave up");
     if (status & IMHD_S_NAN) return fail(IMHD_E_PHYSICS, "non-finite state or max speed: the step is not valid");
     if (status & IMHD_S_ZERO_SPEED) return fail(IMHD_E_PHYSICS, "zero max speed encountered");
-    if (dt_next) *dt_next = host_io[1];
+    if (dt_next) *dt_next = report[0];
     return IMHD_OK;
 }

@@ -75,6 +75,7 @@ struct Scalars {
     unsigned long long cfl_slots[kSlots];
     // flux protection: bad cells found by the predictor (0) and final (1) update
     unsigned int nbad[2];
+    double report[2];                // dt_next and the status bits, for one copy to the host
     // batched driver state (driver.f90:35-186 per box)
     double t, t_end, t_turb, dt_turb_sched;
     long long steps_done, steps_target;
@@ -109,6 +110,10 @@ struct BoxRec {
     int* badlist;
     int badcap;
     short ptws, vec;    // FP32 pair sweeps: x tile of 1 << ptws cell pairs; the rows are whole aligned pairs
+    // a single box (use_one): this step's dt and drive flag, in the launch
+    // parameters; a table's are in each box's Scalars
+    double dt;
+    int drive, pad4_;
 };
 // x pairs of a row, for the FP32 sweeps that take two cells per thread.
 __host__ __device__ inline int pairs_of(int nx) { return (nx + 1) / 2; }
@@ -125,6 +130,7 @@ struct BatchArgs {
     const int* blk2box[kKinds];
     int nbox;
     int use_one;
+    double* report;                  // pinned host memory for a single box's dt_next and status, or null
     BoxRec one;
 };
 
@@ -142,6 +148,7 @@ struct BatchDev {
     int drive_mode = 0;        // 0: no forcing, 1: every box drives (host decided), 2: per-box device flags
     int precision = 64;
     cudaStream_t st = nullptr;
+    bool chain = false;        // the stream's last operation is a kernel of the step being launched
     long long launches = 0;
     bool prof = false;
     cudaEvent_t ev[kStages + 1] = {};
