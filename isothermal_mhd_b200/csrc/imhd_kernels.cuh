@@ -239,8 +239,12 @@ __device__ __forceinline__ void protection_flux(const T* uL, const T* uR, T cs, 
 
 // FP64, and FP32 Roe boxes of a table (five blocks per SM: 96 registers, fewer
 // spill more than the extra warps return); other FP32 boxes run k_pred_flux_f32.
+// FP64 waits on its own arithmetic (2.2 dependency stalls an issue with the 7.7
+// warps that 209 registers leave): three blocks per SM, 168 registers, Roe
+// 464 -> 427 us at 128^3 and 1.89 -> 1.72 ms at 200^3, HLLE 520 -> 409 us at
+// 160^3; four spill more than they return (Roe 435 us).
 template <class T, int SCHEME, bool ONE, bool SHORT = false>
-__global__ void __launch_bounds__(kBX, sizeof(T) == 4 ? 5 : 1)
+__global__ void __launch_bounds__(kBX, sizeof(T) == 4 ? 5 : 3)
 k_pred_flux(BatchArgs ba) {
     step_enter<ONE>();
     constexpr int SOLVER = scheme_solver(SCHEME);
@@ -344,9 +348,10 @@ __device__ __forceinline__ void store_flux(T* __restrict__ F, int D, int n, int 
 // registers; PPM keeps w(a..a+3), the slopes delw(a), delw(a+1) and the right
 // edge of cell a.  Loads stay coalesced along x.  FP64, and FP32 Roe boxes of a
 // table (six blocks per SM, 80 registers, a few spills); other FP32 boxes run
-// k_sweep_f32.
+// k_sweep_f32.  FP64: three blocks per SM as the predictor (Roe + PLM 331 -> 274
+// us at 128^3, HLLD + PPM 399 -> 351).
 template <class T, int SCHEME, int D, bool ONE>
-__global__ void __launch_bounds__(kBX, sizeof(T) == 4 ? 6 : 1) k_corr_flux_march(BatchArgs ba) {
+__global__ void __launch_bounds__(kBX, sizeof(T) == 4 ? 6 : 3) k_corr_flux_march(BatchArgs ba) {
     step_enter<ONE>();
     constexpr int SOLVER = scheme_solver(SCHEME);
     constexpr int RECON = scheme_recon(SCHEME);
@@ -550,9 +555,10 @@ __global__ void __launch_bounds__(TX) k_corr_flux_x(BatchArgs ba) {
 // stages a halo).  PPM evaluates the edges of cells i and i+1 per face.
 // Needs 13 * nx * sizeof(T) bytes of dynamic shared memory.  FP64, and FP32 Roe
 // boxes of a table (eight blocks per SM at 64 registers; six: batched workload
-// 4.67 -> 4.58e9 cell-updates/s); other FP32 boxes run k_xrow_f32.
+// 4.67 -> 4.58e9 cell-updates/s); other FP32 boxes run k_xrow_f32.  FP64: four
+// blocks per SM (Roe + PLM 268 -> 240 us at 128^3, HLLD + PPM 397 -> 273).
 template <class T, int SCHEME, bool ONE>
-__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 8 : 1) k_corr_flux_xrow(BatchArgs ba) {
+__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 8 : 4) k_corr_flux_xrow(BatchArgs ba) {
     step_enter<ONE>();
     constexpr int SOLVER = scheme_solver(SCHEME);
     constexpr int RECON = scheme_recon(SCHEME);
@@ -1172,9 +1178,11 @@ __device__ __forceinline__ CellEV<T> cell_ev(const T* __restrict__ S, int n, int
 // PROT: the corner EMFs of the protection fluxes (Fp -> Ep) of the boxes
 // that compute them, the second compute_cell_corner_emf_3d call of
 // vanleer_mod.f90:336, 396 (the cell-centre EMFs are the same).
-// FP64; FP32 runs k_corner_emf_f32.
+// FP64 (six blocks per SM: 13 long-scoreboard stalls an issue with the three
+// that 134 registers leave; 189 -> 138 us at 128^3, 744 -> 445 at 200^3); FP32
+// runs k_corner_emf_f32.
 template <class T, bool ONE, bool PROT = false, bool SHORT = false>
-__global__ void __launch_bounds__(kBX, 1) k_corner_emf(BatchArgs ba,
+__global__ void __launch_bounds__(kBX, 6) k_corner_emf(BatchArgs ba,
                                                                                        int half_step_state) {
     step_enter<ONE>();
     int local;
@@ -2254,13 +2262,13 @@ __device__ __forceinline__ T vel_of(const T* __restrict__ S, int n, int c, int c
 // 133-157, 204-224, 562-590).
 // A thread walks a column of kSegZ cells along z, carrying the z velocity
 // and the flux through the lower z face (the upper face's of the previous
-// cell: the same operands).  FP64; FP32 runs k_passive_pred_f32.
+// cell: the same operands).  FP64 (eight blocks per SM with up to two scalars:
+// 343 -> 193 us at 200^3 with one); FP32 runs k_passive_pred_f32.
 template <class T, bool ONE, int NP, bool SHORT = false>
-__global__ void __launch_bounds__(kBX, 1) k_passive_pred(BatchArgs ba) {
+__global__ void __launch_bounds__(kBX, NP <= 2 ? 8 : 1) k_passive_pred(BatchArgs ba) {
     step_enter<ONE>();
     int local;
     const BoxRec rp = resolve<ONE>(ba, kKindCellZ, local);
-    const Scalars* sc = rp.sc;
     const int npass = rp.npass;
     if (!rp.active || npass == 0) return;
     const Dims dm = dims_of(rp);
@@ -2349,7 +2357,6 @@ __global__ void __launch_bounds__(kBX, 1) k_passive_corr(BatchArgs ba) {
     step_enter<ONE>();
     int local;
     const BoxRec rp = resolve<ONE>(ba, kKindCellZ, local);
-    const Scalars* sc = rp.sc;
     const int npass = rp.npass;
     if (!rp.active || npass == 0) return;
     const Dims dm = dims_of(rp);
@@ -2470,7 +2477,6 @@ __device__ __forceinline__ V minmod_fast(V wm, V w0, V wp) {
 }
 template <bool ONE, int NP, bool VEC>
 __device__ __forceinline__ void do_passive_pred_f32(const BoxRec& rp, int local) {
-    const Scalars* sc = rp.sc;
     const int npass = rp.npass;
     const Dims dm = dims_of(rp);
     const float* __restrict__ S0 = (const float*)rp.S[0];
@@ -2562,7 +2568,6 @@ __global__ void __launch_bounds__(kBX, NP <= 2 ? 8 : NP <= 4 ? 6 : 3) k_passive_
 
 template <bool ONE, int NP, bool VEC>
 __device__ __forceinline__ void do_passive_corr_f32(const BoxRec& rp, int local) {
-    const Scalars* sc = rp.sc;
     const int npass = rp.npass;
     const Dims dm = dims_of(rp);
     const float* __restrict__ S0 = (const float*)rp.S[0];
@@ -2933,7 +2938,6 @@ __global__ void __launch_bounds__(kTmaTile, 1)
     __shared__ __align__(8) unsigned long long bars[2];
     __shared__ const T* row_src[ppred_rows<NP>()];
     const BoxRec rp = ba.one;
-    const Scalars* sc = rp.sc;
     const int npass = rp.npass;
     if (!rp.active || npass == 0) return;
     const Dims dm = dims_of(rp);

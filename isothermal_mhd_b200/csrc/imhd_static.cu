@@ -46,7 +46,7 @@ namespace {
 
 constexpr size_t kStaticScratchBytes = size_t(48) << 20;   // 48 MiB
 constexpr size_t kScalarsBytes = 4096;                     // imhd::Scalars, rounded up
-constexpr size_t kTableBytes = 4096;                       // box record + block prefixes
+constexpr size_t kTableBytes = 4096;                       // reserved: part of the size limit, unused
 constexpr size_t kPartialBytes = 1024 * 6 * 8;             // reduction partials (unused: no forcing)
 constexpr int kMaxDevices = 64;
 
@@ -80,8 +80,6 @@ extern "C" int imhd_step_static(int precision, int nx, int ny, int nz, int riema
                                 double cour, const void* state_in, void* state_out, double dt, double* dt_next,
                                 void* stream) {
     static_assert(sizeof(imhd::Scalars) <= kScalarsBytes, "scalar block outgrew its scratch slot");
-    static_assert(256 + sizeof(int) * imhd::kKinds * 2 <= kTableBytes && sizeof(imhd::BoxRec) <= 256,
-                  "box table outgrew its scratch slot");
     auto fail = [](int code, const std::string& m) { imhd::set_last_error(code, m.c_str()); return code; };
     if (precision != 32 && precision != 64) return fail(IMHD_E_ARG, "precision must be 32 or 64");
     if (nx < 4 || ny < 4 || nz < 4) return fail(IMHD_E_ARG, "every edge needs at least 4 cells");
@@ -114,8 +112,7 @@ extern "C" int imhd_step_static(int precision, int nx, int ny, int nz, int riema
     rec.S[0] = const_cast<void*>(state_in);
     rec.S[1] = state_out;
     unsigned char* p = base;
-    rec.sc = (imhd::Scalars*)p;  p += kScalarsBytes;
-    unsigned char* table = p;    p += kTableBytes;
+    rec.sc = (imhd::Scalars*)p;  p += kScalarsBytes + kTableBytes;
     rec.partials = (double*)p;   p += kPartialBytes;
     rec.F = p;  p += align256(18 * n * esz);
     rec.E = p;  p += align256(3 * n * esz);

@@ -227,44 +227,40 @@ inline void init_rec(BoxRec& r, int nx, int ny, int nz, int npass, int riemann, 
     r.active = 1;
 }
 
-// Relative time of a single-box launch of `threads` columns of `len` cells
-// (blocks of kBX threads, `occ` of them resident per SM): `len` cells plus
-// `start` for what a column loads and computes before its first cell, times
-// the blocks that an SM takes one after the other.  A last wave of r blocks
-// per SM costs at least `fill` blocks' time (fewer leave the SM waiting on
-// latency).
-inline double column_cost(long blocks_per_unit, int len, double start, int occ, int fill) {
-    const long k = (blocks_per_unit / len + 147) / 148;
-    const long r = k % occ;
-    return (len + start) * (double)((k - r) + (r == 0 ? 0 : r < fill ? fill : r));
+// Relative time of a single-box sweep whose columns of one cell would be
+// `units` blocks, run as columns of `len` cells: `len` cells plus 0.6 for the
+// slope that a column computes before its first face, times the blocks that an
+// SM takes (148 SMs, `occ` blocks resident; fewer leave it waiting on latency,
+// and a last wave that does not fill costs a part of its idle slots).
+inline double column_cost(long units, int len, int occ) {
+    const long k = (units / len + 147) / 148, r = k % occ;
+    return (len + 0.6) * (k <= occ ? (double)occ : (double)k + (r ? 0.3 * (double)(occ - r) : 0.0));
 }
 // Column lengths of a single box (a table shares its launches between boxes
 // and keeps the lengths of init_rec).  The y / z sweeps take the length of
-// least column_cost; the z-column kernels keep kSegZ planes (whose loops the
-// compiler unrolls) unless those leave fewer than 8 blocks per SM.  Measured
-// per step, Roe + PLM with scalars, all lengths 16 (as every box had), 8, 4,
-// 2, 1 (us between events): FP32 32^3 227, 163, 122, 102, 90; 64^3 306, 212,
-// 163, 169, 163; 96^3 373, 318, 320, 337, 365; 128^3 627, 616, 605, 652, 725;
-// 192^3 1827, 1932, 1987 (16 stays); FP64 64^3 577, 375, 385, 372, 393; 96^3
-// 1044, 953, 983, 1052, 1202; 128^3 2154, 2020, 2093; 192^3 7135, 7176.
+// least column_cost.  The z-column kernels take the longest columns, up to
+// kSegZ planes, that leave 5 blocks per SM in FP32 (tiles of cell pairs) and
+// 6.5 in FP64, where boxes below 168^3 stop at 8 planes.  Measured, us a step
+// with the lengths as every box had them (16), with these, and with the best
+// pair found: FP32 Roe 32^3 140, 63, 61; 64^3 149, 90, 85; 80^3 204, 145, 141;
+// 96^3 258, 196, 193; 128^3 390, 381, 378; 160^3 721, 725, 715; FP64 Roe 32^3
+// 490, 105, 104; 48^3 533, 194, 194; 64^3 646, 323, 318; 96^3 926, 832, 825;
+// 128^3 2037, 1851, 1830.
 inline void one_box_segments(BoxRec& r, size_t esz) {
-    const bool pairs = pair_sweeps(r, esz, true);
-    const int tws = pairs ? r.ptws : r.tws, nu = pairs ? pairs_of(r.nx) : r.nx, th = kBX >> tws;
-    const int occ = esz == 8 ? 2 : 6, fill = esz == 8 ? 2 : 4, socc = pairs ? 3 : occ, sfill = pairs ? 2 : fill;
-    const long sweep = ceil_div(nu, 1 << tws) *
-                       ((long)ceil_div(r.nz, th) * r.ny + (long)ceil_div(r.ny, th) * r.nz) / 2;
-    const long cols = (long)ceil_div(r.nx, 1 << r.tws) * ceil_div(r.ny, kBX >> r.tws) * r.nz;
+    const bool sp = pair_sweeps(r, esz, true);
+    auto units = [&](bool pairs, int d) {       // blocks of one-cell columns along axis d
+        const int tws = pairs ? r.ptws : r.tws, nu = pairs ? pairs_of(r.nx) : r.nx, th = kBX >> tws;
+        return (long)ceil_div(nu, 1 << tws) * (d == 1 ? (long)ceil_div(r.nz, th) * r.ny : (long)ceil_div(r.ny, th) * r.nz);
+    };
+    const long sweep = (units(sp, 1) + units(sp, 2)) / 2, cols = units(esz == 4, 2);
     double best = 0.0;
     for (int s = 0; s <= 5; ++s) {
-        const double c = column_cost(sweep, 1 << s, 0.6, socc, sfill);
+        const double c = column_cost(sweep, 1 << s, esz == 8 || sp ? 3 : 6);
         if (s == 0 || c <= best) { best = c; r.segs = s; }
     }
-    if (cols < 8L * 148 * kSegZ) {
-        for (int s = 0; s <= kSegZLog; ++s) {
-            const double c = column_cost(cols, 1 << s, 0.5, occ, fill);
-            if (s == 0 || c <= best) { best = c; r.segzs = s; }
-        }
-    }
+    const long least = esz == 8 ? 962 : 740;
+    r.segzs = esz == 8 && cols < 37888 ? kSegZLog - 1 : kSegZLog;
+    while (r.segzs > 0 && (cols >> r.segzs) < least) --r.segzs;
 }
 
 // Device bytes of one box's buffers (state x2, fluxes, EMFs, half-step
