@@ -766,17 +766,26 @@ __device__ __forceinline__ void pred_flux_f32(const BoxRec& rp, int local, bool 
             ld_fields_any(S, n, all, row + x0 + k0 * plane, row + x1 + k0 * plane, vec, u);
             to_cell(u, cur);
         }
+        constexpr bool AHEAD = SOLVER == 2 || SOLVER == 3;
+        float e[6];                            // the cell after the pair
+        auto after = [&](int kp, float* o) {
+            const int fe[6] = {0, 1, 2, 3, 5, 6};
+#pragma unroll
+            for (int m = 0; m < 6; ++m) o[m] = __ldg(fld(S, fe[m], n) + (row + x2 + kp));
+        };
+        if (AHEAD) after(k0 * plane, e);
         for (int k = k0; k < k1; ++k) {
             const int kp = k * plane, kz = wrap_up(k, dm.nz) * plane, c0 = row + x0 + kp, c1 = row + x1 + kp;
             F2 sdrop = smax;     // faces outside zlo..zhi-1 do not enter smax
             F2& sref = (k >= rp.zlo && k < rp.zhi) ? smax : sdrop;
-            // this plane's y row and the plane above, loaded before the x face
-            float e[6];
+            // this plane's y row and the plane above (and, AHEAD, the cell
+            // after the pair there), loaded before the x face
+            float en[6];
             F2 u[6], z[10];
             {
-                const int f[6] = {0, 1, 2, 3, 5, 6}, fy[6] = {0, 1, 2, 3, 4, 6};
-#pragma unroll
-                for (int m = 0; m < 6; ++m) e[m] = __ldg(fld(S, f[m], n) + (row + x2 + kp));
+                const int fy[6] = {0, 1, 2, 3, 4, 6};
+                if (!AHEAD) after(kp, e);
+                else after(kz, en);
                 if (vec) {
                     ld_fields<true>(S, n, fy, rowp + x0 + kp, rowp + x1 + kp, u);
                     ld_fields<true>(S, n, all, row + x0 + kz, row + x1 + kz, z);
@@ -816,13 +825,19 @@ __device__ __forceinline__ void pred_flux_f32(const BoxRec& rp, int local, bool 
             cell_side<2, 0, 1>(up, R);
             face_fast<SOLVER>(L, R, cur.bf[2], cs, asqr, sref, rp, 2, c0, c1, vec, two);
             cur = up;
+            if (AHEAD) {
+#pragma unroll
+                for (int m = 0; m < 6; ++m) e[m] = en[m];
+            }
         }
     }
     block_atomic_max<kBX>(rp.sc->smax_slots, (double)top_lane(smax));
 }
 // Roe: one body per row alignment, which the compiler schedules better (438
 // against 479 us at 256^3); HLLD and HLLE: one body that tests it at each
-// group of loads (492 against 530 us).
+// group of loads (492 against 530 us), with the cell after the pair loaded a
+// plane ahead, whose face comes first (HLLD 496 -> 465, HLLE 384 -> 366; Roe
+// loses, 440 -> 446).
 template <int SOLVER, bool ONE>
 __global__ void __launch_bounds__(kBX, 3) k_pred_flux_f32(BatchArgs ba, int kind) {
     step_enter<ONE>();
