@@ -2581,6 +2581,16 @@ __global__ void __launch_bounds__(kBX, NP <= 2 ? 8 : NP <= 4 ? 6 : 3) k_passive_
     else do_passive_pred_f32<ONE, NP, false>(rp, local);
 }
 
+// Line of *p brought into L2, for a load some planes later.
+__device__ __forceinline__ void l2_ahead(const float* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
+// Bound by the latency of its loads (256^3, 2 scalars: long scoreboard 6 per
+// issue at 32% of DRAM peak, 96 registers for 5 blocks per SM).  What a pair
+// is the first to read of a plane, its own v_x, v_y and step-start scalars
+// and, ahead by its z stencil, v_z and the half-step scalars, is brought into
+// L2 two planes before its load, without registers: 239 -> 187 us there, 4
+// scalars at 320^3 968 -> 708, 128^3 38 -> 34, 64^3 the same.  The same loads
+// into registers a plane ahead: 203 and 782 us; with 6 (4) blocks 224 and 937.
 template <bool ONE, int NP, bool VEC>
 __device__ __forceinline__ void do_passive_corr_f32(const BoxRec& rp, int local) {
     const int npass = rp.npass;
@@ -2632,6 +2642,19 @@ __device__ __forceinline__ void do_passive_corr_f32(const BoxRec& rp, int local)
     }
 #pragma unroll 1
     for (int k = k0; k < k1; ++k) {
+        {
+            const int k2 = wrap_up(wrap_up(k, dm.nz), dm.nz), k3 = wrap_up(k2, dm.nz);
+            const int f2 = row + x0 + k2 * plane, f3 = row + x0 + k3 * plane;
+            l2_ahead(VT + f2);
+            l2_ahead(VT + n + f2);
+            l2_ahead(VZ + f3);
+#pragma unroll
+            for (int q = 0; q < NP; ++q) {
+                const size_t s = (size_t)min(q, npass - 1);
+                l2_ahead(S0 + (10 + s) * n + f2);
+                l2_ahead(SH + s * n + f3);
+            }
+        }
         const int kp = k * plane, kz = wrap_up(k, dm.nz) * plane, kz2 = wrap_up(wrap_up(k, dm.nz), dm.nz) * plane;
         const int c0 = row + x0 + kp, c1 = row + x1 + kp;
         const F2 vx0 = ld_lanes<F2, VEC>(VT, c0, c1), vy0 = ld_lanes<F2, VEC>(VT + n, c0, c1);
