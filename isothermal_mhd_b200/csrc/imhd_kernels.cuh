@@ -2589,7 +2589,9 @@ __device__ __forceinline__ void l2_ahead(const float* p) { asm volatile("prefetc
 // is the first to read of a plane, its own v_x, v_y and step-start scalars
 // and, ahead by its z stencil, v_z and the half-step scalars, is brought into
 // L2 two planes before its load, without registers: 239 -> 187 us there, 4
-// scalars at 320^3 968 -> 708, 128^3 38 -> 34, 64^3 the same.  The same loads
+// scalars at 320^3 968 -> 708, 128^3 38 -> 34; a single box below a million
+// cells, whose fields L2 holds, only pays for it (101 x 83 x 67: 1065 -> 1076
+// us for six steps) and goes without.  The same loads
 // into registers a plane ahead: 203 and 782 us; with 6 (4) blocks 224 and 937.
 template <bool ONE, int NP, bool VEC>
 __device__ __forceinline__ void do_passive_corr_f32(const BoxRec& rp, int local) {
@@ -2640,9 +2642,10 @@ __device__ __forceinline__ void do_passive_corr_f32(const BoxRec& rp, int local)
                 fz_m[q] = upwind_pick(sm + dm_, s_0[q] - d0, half * (vz_m + vz_0));
             }
     }
+    const bool far = !ONE || n >= 1 << 20;
 #pragma unroll 1
     for (int k = k0; k < k1; ++k) {
-        {
+        if (far) {
             const int k2 = wrap_up(wrap_up(k, dm.nz), dm.nz), k3 = wrap_up(k2, dm.nz);
             const int f2 = row + x0 + k2 * plane, f3 = row + x0 + k3 * plane;
             l2_ahead(VT + f2);
