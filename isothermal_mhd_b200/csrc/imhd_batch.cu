@@ -442,7 +442,7 @@ bool next_candidate(imhd_batch* x, int& tile, int& segs, int& segzs) {
             tile = x->best_tile; segzs = x->best_segzs; segs = kLogs[x->tune_idx];
             return true;
         }
-        if (x->tune_stage == 1) {          // reserved (z column length: compile-time)
+        if (x->tune_stage == 1) {          // reserved (z column length: every table keeps init_rec's)
             x->tune_stage = 2;
             x->tune_idx = 0;
             continue;

@@ -42,14 +42,20 @@ inline int pair_tile(int nx, int tws) {
     return best;
 }
 
+// Planes that a thread of a z-column kernel walks: 1 << segzs in the kernels that
+// take two cells per thread and in a single box's, kSegZ in a table's one-cell
+// kernels, which have the length at compile time (decode_cellz).
+inline int column_planes(const BoxRec& r, bool pairs, bool single) { return pairs || single ? 1 << r.segzs : kSegZ; }
+
 // Blocks of box r for decomposition `kind`.
 inline long blocks_of(const BoxRec& r, int kind, size_t esz, bool row_pairs, bool single) {
     const int tw = 1 << r.tws, th = kBX >> r.tws;
     long nbx = ceil_div(r.nx, tw), nby = ceil_div(r.ny, th), nbz = ceil_div(r.nz, th);
     if (kind == kKindCell) return nbx * nby * r.nz;
-    if (kind == kKindCellZ) return esz == 4 ? 0 : nbx * nby * ceil_div(r.nz, 1 << r.segzs);
+    if (kind == kKindCellZ) return esz == 4 ? 0 : nbx * nby * ceil_div(r.nz, column_planes(r, false, single));
     if (kind == kKindPairZ)
-        return esz == 4 ? (long)ceil_div(pairs_of(r.nx), 1 << r.ptws) * ceil_div(r.ny, kBX >> r.ptws) * ceil_div(r.nz, 1 << r.segzs)
+        return esz == 4 ? (long)ceil_div(pairs_of(r.nx), 1 << r.ptws) * ceil_div(r.ny, kBX >> r.ptws) *
+                              ceil_div(r.nz, column_planes(r, true, single))
                         : 0;
     if (kind == kKindRed) return r.nred;
     if (esz == 4 && (kind == kKindUpdTma || kind == kKindUpdTma64)) return 0;   // FP64 kernels
@@ -69,7 +75,7 @@ inline long blocks_of(const BoxRec& r, int kind, size_t esz, bool row_pairs, boo
         nbz = ceil_div(r.nz, kBX >> r.ptws);
     }
     switch (sub) {
-        case kSubCell: return nbx * nby * ceil_div(r.nz, 1 << r.segzs);   // z columns of the predictor fluxes
+        case kSubCell: return nbx * nby * ceil_div(r.nz, column_planes(r, pair_fluxes(r, esz, single), single));   // z columns of the predictor fluxes
         case kSubXRow: return row ? (long)(row_pairs && pairs ? ceil_div(r.ny, 2) : r.ny) * r.nz : 0;
         case kSubXTile: return row ? 0 : (long)ceil_div(r.nx, kTX) * r.ny * r.nz;
         case kSubMarchY: return nbx * nbz * ceil_div(r.ny, 1 << r.segs);   // (x, z) tiles marching along y

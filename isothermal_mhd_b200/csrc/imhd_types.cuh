@@ -92,7 +92,8 @@ struct BoxRec {
     int zlo, zhi;           // z planes whose cells and faces enter the step's maxima and sums
     int tws, protect;       // x width of the cell tiles is 1 << tws (32, 64 or 128), height kBX >> tws;
                             // protect: HLLE protection fluxes of a Roe box (flux_protection)
-    int segs, segzs;        // faces per thread of the y / z sweeps 1 << segs; segzs == kSegZLog (reserved)
+    int segs, segzs;        // faces per thread of the y / z sweeps 1 << segs, planes per thread of the z-column
+                            // kernels 1 << segzs (a table's one-cell kernels: kSegZ, see column_planes)
     double dx, cs, cour, edot, dt_turb;
     void* S[2];
     void* F;        // 18 flux fields
