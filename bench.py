@@ -214,13 +214,14 @@ def stage_bytes(esz, npass):
 
 
 # DRAM bytes per cell of one launch (dram__bytes_read.sum + dram__bytes_write.sum over the cells of the
-# launch) from an ncu capture at 256^3 of the same kernel and scheme; traffic grows with the cell count,
-# so a launch at n^3 moves about n^3 times this.  Keyed by (stage, precision, riemann, recon).
+# launch) from an ncu capture at 256^3 with two scalars of the kernel that the stage runs
+# (profiles/pair_kernels_fp32_256.md); traffic grows with the cell count, so a launch at n^3 moves about
+# n^3 times this.  Keyed by (stage, precision, riemann, recon).
 NCU_TRAFFIC_PER_CELL = {
-    ("pred_flux", 32, "roe", "plm"): (677.4e6 + 1161.1e6) / 256 ** 3,
-    # the update does not depend on the solver or the reconstruction (mean of the two launches of a step;
-    # the final one also writes the passive corrector's three velocities)
-    ("update", 32): (1493.0e6 + 644.8e6 + 1494.1e6 + 840.3e6) / 2 / 256 ** 3,
+    ("pred_flux", 32, "roe", "plm"): 110.1,
+    # k_update_f32, which does not depend on the solver or the reconstruction (mean of the two launches of
+    # a step; the final one also writes the passive corrector's three velocities)
+    ("update", 32): (127.4 + 139.3) / 2,
 }
 
 # step stages that are launches of one kernel: the roofline reports the kernel
