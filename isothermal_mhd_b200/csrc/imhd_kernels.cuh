@@ -1312,12 +1312,11 @@ __global__ void __launch_bounds__(kBX, 6) k_corner_emf(BatchArgs ba,
 // neighbour of the first, so a pair evaluates 2 + 1 cells of each of its two
 // rows per plane where two threads evaluated 6, every load of a row is 8
 // bytes.  The upwinded differences are selected after they are subtracted (both
-// halves take the same side); in a table the results are those of k_corner_emf
-// compiled for float, to the bit.  Bound
-// by memory latency and bandwidth: 2.24 -> 1.57 ms at 512^3, 5.5 TB/s of the
-// algorithmic 64 B per cell (70% of DRAM peak in ncu at 256^3), with one body
-// per row alignment so that a plane's loads leave together (a test at each
-// group of loads: 2.51 ms); three or five blocks per SM: 1.80, 1.76 ms.
+// halves take the same side).  Bound by memory latency and bandwidth: 2.24 ->
+// 1.57 ms at 512^3, 5.5 TB/s of the algorithmic 64 B per cell (68% of DRAM peak
+// in ncu at 256^3), with one body per row alignment so that a plane's loads
+// leave together (a test at each group of loads: 2.51 ms); three or five blocks
+// per SM: 1.80, 1.76 ms.
 template <class V>
 struct CellE {
     V ex, ey, ez, ux, uy, uz;    // cell-centre EMF (ecc3) and velocity
@@ -1437,8 +1436,10 @@ __device__ __forceinline__ void do_corner_emf_f32(const BoxRec& rp, int local, i
         ld_fields<VEC>(F, n, fx, r2 + kp, 0, wx);
         const F2 neg = same<F2>(-1.0f), quarter = same<F2>(0.25f);
         // Only the signs of the face velocities are used.  In a table, where one
-        // is near zero, the velocities are divided out as k_corner_emf divides,
-        // so that the same side is taken (0.14 ms more at 512^3).
+        // is near zero, the velocities are divided out as the one-cell FP32
+        // kernel divided them (0.14 ms more at 512^3): the same side is then
+        // taken but in about one Roe box of 110 (imhd_physics_table.cuh), where
+        // the side differs at one edge.
         F2 vx = A.a.ux + A.xux, vy = A.a.uy + A.buy, vz = A.a.uz + B.a.uz;
         const float tol = ONE ? 0.0f : 1.0e-6f;
         const bool near = near_zero(A.a.ux, A.xux, tol) || near_zero(A.a.uy, A.buy, tol) || near_zero(A.a.uz, B.a.uz, tol);

@@ -261,10 +261,6 @@ static void ensure_passive_tma_attr() {
     }
 }
 
-// Passive corrector: the bulk-copy fed kernel for a single box whose rows
-// are whole 128-cell tiles (16-byte aligned rows of every field it streams),
-// the z-column kernel otherwise; scalar arrays sized for the table's largest
-// passive count.
 template <class T>
 static void ensure_passive_pred_tma_attr() {
     static bool attr_set[64] = {};   // per precision and device
@@ -325,6 +321,10 @@ static void launch_passive_pred(BatchDev& b, dim3 gz) {
     }
 }
 
+// Passive corrector: FP32 the pair kernel; FP64 the bulk-copy fed kernel for a
+// single box whose rows are whole 128-cell tiles (16-byte aligned rows of every
+// field it streams), the z-column kernel otherwise; scalar arrays sized for the
+// table's largest passive count.
 template <class T, bool ONE>
 static void launch_passive_corr(BatchDev& b, dim3 gz) {
     const BoxRec& r = b.a.one;

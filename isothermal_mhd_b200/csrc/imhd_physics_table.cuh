@@ -5,10 +5,17 @@
 // 0.3 to 0.65, vanleer_mod.f90:2829-2833), so a single-precision result that
 // rounds differently takes the other branch at an interface now and then: on a
 // 32^3 box of rms Mach 1 about once in 150 steps, and the cell beside it moves
-// by up to 5e-4.  A batch or a served request makes hundreds of steps, so its
-// Roe boxes keep one arithmetic, this one (contracted by the compiler), and
-// reproduce what they gave before the single boxes took pairs of interfaces
-// (imhd_physics_fast.cuh); HLLD and HLLE have no such jump and use the pairs.
+// by up to 5e-4.  This is the arithmetic (contracted by the compiler) that all
+// FP32 boxes had before the single ones took pairs of interfaces
+// (imhd_physics_fast.cuh); the Roe boxes of a table keep it so that a batch or a
+// served request gives what it gave: 674 of 680 such boxes (32^3 to 64^3, rms
+// Mach 1 and 2, 8 to 48 steps) to the bit, the others but for an upwind side of
+// the corner EMF (2e-5).  It is no more accurate than the pairs: over 200 32^3
+// boxes of 8 steps the mean relative L1 error against FP64 is the same within
+// 2%, and the largest error of a cell passes 1e-5 in 27 boxes of a table, 26
+// single ones and 35 single ones with this arithmetic.  So a Roe box of a table and the
+// same box alone agree to rounding but for such a cell now and then.  HLLD and
+// HLLE have no jump and use the pairs in tables too.
 #pragma once
 
 #include "imhd_physics.cuh"

@@ -46,7 +46,7 @@ namespace {
 
 constexpr size_t kStaticScratchBytes = size_t(48) << 20;   // 48 MiB
 constexpr size_t kScalarsBytes = 4096;                     // imhd::Scalars, rounded up
-constexpr size_t kTableBytes = 4096;                       // reserved: part of the size limit, unused
+constexpr size_t kTableBytes = 4096;                       // unused, but part of the size limit: the sizes accepted stay the same
 constexpr size_t kPartialBytes = 1024 * 6 * 8;             // reduction partials (unused: no forcing)
 constexpr int kMaxDevices = 64;
 

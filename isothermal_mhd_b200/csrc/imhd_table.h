@@ -109,6 +109,11 @@ inline bool build_prefix(const std::vector<BoxRec>& recs, size_t esz, std::vecto
     bd.row_nx_max = 0;
     for (const BoxRec& r : recs)
         if (row_capable(r.nx, esz) && r.nx > bd.row_nx_max) bd.row_nx_max = r.nx;
+    // Two rows per block wherever they fit, although fewer blocks then share an
+    // SM as the rows grow (four at 512 cells, two from 768).  A Roe step of (nx,
+    // 96, 96) with the one-cell kernels everywhere and with pairs, us: 512 951,
+    // 723; 640 1186, 934; 768 1345, 1099; 896 1585, 1300; 944 1857, 1389; and of
+    // (946, 64, 64), whose x rows go one by one: 976, 794.
     bd.row_pairs = esz == 4 && 2 * 13 * (size_t)bd.row_nx_max * esz <= kRowSmemMax;
     prefix.assign((size_t)kKinds * (nbox + 1), 0);
     for (int k = 0; k < kKinds; ++k) {

@@ -4,10 +4,15 @@
 //
 // The FP32 sweeps are bound by instruction issue, and one packed instruction
 // (add/sub/mul/fma.rn.f32x2) does the work of two scalar ones in one issue
-// slot; it takes the FP32 pipe as long as the two would.  Every operation is
-// rounded separately and fused multiply-adds are written out (fma), so that
-// the compiler contracts nothing by itself: the same expression gives the same
-// bits in F1 and F2, in every kernel and in every copy that inlining makes.
+// slot; it takes the FP32 pipe as long as the two would.  Every operation on
+// F1 and F2 is rounded separately and fused multiply-adds are written out
+// (fma), so that the compiler contracts nothing by itself: the same expression
+// gives the same bits in F1 and F2, in every kernel and in every copy that
+// inlining makes.  That covers PLM.  The PPM edges and the primitive-variable
+// limiters are written on plain floats (imhd_physics.cuh) in a unit compiled
+// with contraction, and so are the FP64 eigenvector normalisations near the
+// triple point: a column's first cells and its loop are separate copies of
+// them, so FP32 PPM may differ in the last bit with the column length.
 // What has no packed form (reciprocals, roots, minima, selections) runs on the
 // halves.
 #pragma once
