@@ -9,8 +9,9 @@
 // FP32 boxes had before the single ones took pairs of interfaces
 // (imhd_physics_fast.cuh); the Roe boxes of a table keep it so that a batch or a
 // served request gives what it gave: 674 of 680 such boxes (32^3 to 64^3, rms
-// Mach 1 and 2, 8 to 48 steps) to the bit, the others but for an upwind side of
-// the corner EMF (2e-5).  It is no more accurate than the pairs: over 200 32^3
+// Mach 1 and 2, 8 to 48 steps) to the bit; of the other six the four that were
+// followed step by step took another upwind side of the corner EMF at one edge
+// (2e-5).  It is no more accurate than the pairs: over 200 32^3
 // boxes of 8 steps the mean relative L1 error against FP64 is the same within
 // 2%, and the largest error of a cell passes 1e-5 in 27 boxes of a table, 26
 // single ones and 35 single ones with this arithmetic.  So a Roe box of a table and the
